@@ -65,22 +65,73 @@ int fail(swift_ctx* ctx, int code, const std::string& msg) {
       return fail(ctx, SWIFT_E_CUDA, std::string("kernel launch: ") + cudaGetErrorString(e_)); \
   } while (0)
 
-// Stream-ordered temporaries released at the end of a call.
+// Stream-ordered temporaries released at the end of a call.  Requests up to
+// kCarve bytes are cut from shared blocks: a call makes about 60 of them, and
+// a pool allocation with its release costs the host some 4 us each, a third
+// of a one-read call.
 struct Scratch {
+  static constexpr size_t kCarve = 1u << 20, kBlock = 4u << 20;
   cudaStream_t st;
   std::vector<void*> ptrs;
+  char* block = nullptr;
+  size_t left = 0;
   explicit Scratch(cudaStream_t s) : st(s) {}
   ~Scratch() {
     for (void* p : ptrs) cudaFreeAsync(p, st);
   }
   template <typename T>
   cudaError_t get(T** out, size_t count) {
+    // 256-byte steps, as a pool allocation is aligned
+    const size_t bytes = (std::max<size_t>(count * sizeof(T), 16) + 255) & ~(size_t)255;
+    if (bytes <= kCarve && bytes <= left) {
+      *out = (T*)block;
+      block += bytes;
+      left -= bytes;
+      return cudaSuccess;
+    }
     void* p = nullptr;
-    cudaError_t e = cudaMallocAsync(&p, std::max<size_t>(count * sizeof(T), 16), st);
+    const bool carve = bytes <= kCarve;
+    cudaError_t e = cudaMallocAsync(&p, carve ? kBlock : bytes, st);
     if (e != cudaSuccess) return e;
     ptrs.push_back(p);
     *out = (T*)p;
+    if (carve) {
+      block = (char*)p + bytes;
+      left = kBlock - bytes;
+    }
     return cudaSuccess;
+  }
+};
+
+// Small device values the host waits for.  A copy to pageable memory holds
+// the host up by itself; these land in the context's pinned buffer and are
+// handed out by sync(), the one wait.  One object at a time, from its first
+// get() to its sync().
+struct Readback {
+  struct Item {
+    void* dst;
+    const char* at;
+    size_t bytes;
+  };
+  swift_ctx* ctx;
+  std::vector<Item> items;
+  size_t used = 0;
+  explicit Readback(swift_ctx* c) : ctx(c) {}
+  cudaError_t get(void* dst, const void* src, size_t bytes) {
+    if (!ctx->mail || used + bytes > kMailBytes)
+      return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, ctx->st);
+    char* at = ctx->mail + used;
+    used += (bytes + 15) & ~(size_t)15;
+    items.push_back({dst, at, bytes});
+    return cudaMemcpyAsync(at, src, bytes, cudaMemcpyDeviceToHost, ctx->st);
+  }
+  cudaError_t sync() {
+    const cudaError_t e = cudaStreamSynchronize(ctx->st);
+    if (e == cudaSuccess)
+      for (const Item& i : items) memcpy(i.dst, i.at, i.bytes);
+    items.clear();
+    used = 0;
+    return e;
   }
 };
 
@@ -127,16 +178,15 @@ struct TextChunks {
   int n_chunks = 1;
   uint64_t rec_at[kOutChunks + 1] = {}, text_at[kOutChunks + 1] = {};
   // Queues the copies of the range starts' text offsets (offs: exclusive
-  // scan of the record sizes); they hold after the caller's next
-  // synchronisation of st.
-  int plan(swift_ctx* ctx, cudaStream_t st, const uint64_t* offs, int64_t n, bool to_host) {
+  // scan of the record sizes); they hold after rb.sync().
+  int plan(swift_ctx* ctx, Readback& rb, const uint64_t* offs, int64_t n, bool to_host) {
     n_chunks = to_host && n >= kOutChunkMin ? kOutChunks : 1;
     for (int c = 0; c <= n_chunks; ++c) rec_at[c] = (uint64_t)n * c / n_chunks;
     for (int c = 1; c < n_chunks; ++c)
-      CK(cudaMemcpyAsync(&text_at[c], offs + rec_at[c], 8, cudaMemcpyDeviceToHost, st));
+      CK(rb.get(&text_at[c], offs + rec_at[c], 8));
     return SWIFT_OK;
   }
-  // After that synchronisation: the write kernels into text (total bytes),
+  // After that: the write kernels into text (total bytes),
   // `done` recorded on st after the last one.  The text goes to host_out
   // when it fits host_cap; the copies are complete once st is synchronised.
   int write(swift_ctx* ctx, cudaStream_t st, FormatArgs fa, bool sam, char* text, uint64_t total,
@@ -542,8 +592,9 @@ int seed_ssaha(swift_ctx* ctx, Scratch& sc, SeedArgs a, SeedOut* out) {
   CK(cudaEventRecord(ctx->ev[10], st));
   out->launches += n > 0 ? 3 : 0;
   int32_t h_novl = 0;
-  CK(cudaMemcpyAsync(&h_novl, novl, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-  CK(cudaStreamSynchronize(st));
+  Readback rb(ctx);
+  CK(rb.get(&h_novl, novl, sizeof(int32_t)));
+  CK(rb.sync());
   if (n > 0) {
     float t = 0;
     cudaEventElapsedTime(&t, ctx->ev[9], ctx->ev[10]);
@@ -698,8 +749,9 @@ int run_seed(swift_ctx* ctx, const swift_index* idx, const swift_reads* rd, int 
     CKLAUNCH();
     out->launches += ns > 0 ? 1 : 0;
     int32_t h_novl = 0;
-    CK(cudaMemcpyAsync(&h_novl, novl, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
+    Readback rb(ctx);
+    CK(rb.get(&h_novl, novl, sizeof(int32_t)));
+    CK(rb.sync());
     out->overflow = h_novl;
     if (h_novl > 0) {  // strands redone with the reference's full array sizes
       s13.list = ovl;
@@ -768,8 +820,9 @@ int run_seed(swift_ctx* ctx, const swift_index* idx, const swift_reads* rd, int 
     CKLAUNCH();
     ++out->launches;
     std::vector<uint64_t> rec0(W + 1);
-    CK(cudaMemcpyAsync(rec0.data(), d_rec0, (W + 1) * 8, cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
+    Readback rb(ctx);
+    CK(rb.get(rec0.data(), d_rec0, (W + 1) * 8));
+    CK(rb.sync());
     const uint64_t total = rec0[W];
     for (size_t r = 0; r < W; ++r) {
       (*wave)[r].rec0 = (int64_t)rec0[r];
@@ -802,16 +855,16 @@ int run_seed(swift_ctx* ctx, const swift_index* idx, const swift_reads* rd, int 
   out->launches += (n > 0 ? 1 : 0) + exclusive_scan_u64(st, cnt, roff, n, tmp, tot_d);
   CKLAUNCH();
   uint64_t total_in = 0;
-  CK(cudaMemcpyAsync(&total_in, tot_d, sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
+  Readback rb(ctx);
+  CK(rb.get(&total_in, tot_d, sizeof(uint64_t)));
   // the stale trailing batch of searchQueries3; search2Queries has none
   const std::vector<int32_t> no_rep;
   const std::vector<int32_t>& rep = seeder == 1 ? no_rep : rd->repeats;
   std::vector<uint64_t> rep_cnt(rep.size()), rep_off(rep.size());
   std::vector<int32_t> rep_nb(2 * rep.size());
   for (size_t i = 0; i < rep.size(); ++i)
-    CK(cudaMemcpyAsync(&rep_nb[2 * i], nbest + 2 * (int64_t)rep[i], 2 * sizeof(int32_t),
-                       cudaMemcpyDeviceToHost, st));
-  CK(cudaStreamSynchronize(st));
+    CK(rb.get(&rep_nb[2 * i], nbest + 2 * (int64_t)rep[i], 2 * sizeof(int32_t)));
+  CK(rb.sync());
   uint64_t total = total_in;
   for (size_t i = 0; i < rep.size(); ++i) {
     rep_off[i] = total;
@@ -860,6 +913,7 @@ int upload_reads(swift_ctx* ctx, const char* b, size_t len, swift_reads** out,
   if (transient) r->pool_st = st;
   auto t0 = std::chrono::steady_clock::now();
   auto bail = [&](int code, const std::string& m) {
+    cudaStreamSynchronize(st);  // the caller's bytes may still be copied from
     swift_reads_destroy(r);
     return fail(ctx, code, m);
   };
@@ -869,10 +923,11 @@ int upload_reads(swift_ctx* ctx, const char* b, size_t len, swift_reads** out,
     if (e_ != cudaSuccess) return bail(SWIFT_E_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_)); \
   } while (0)
   CKR(transient ? cudaMallocAsync(&r->d_bytes, len + 64, st) : cudaMalloc(&r->d_bytes, len + 64));
+  // (the copy is timed by events, so the host need not wait for it alone)
+  CKR(cudaEventRecord(ctx->ev[10], st));
   CKR(cudaMemcpyAsync(r->d_bytes, b, len, cudaMemcpyHostToDevice, st));
-  CKR(cudaStreamSynchronize(st));
-  if (h2d_ms) *h2d_ms = ms_since(t0);
-  t0 = std::chrono::steady_clock::now();
+  CKR(cudaEventRecord(ctx->ev[11], st));
+  float copy_ms = 0;
   {
     Scratch sc(st);
     const uint64_t tiles = parse_tiles(len);
@@ -893,8 +948,10 @@ int upload_reads(swift_ctx* ctx, const char* b, size_t len, swift_reads** out,
     exclusive_scan_u32(st, cnt, off, (int64_t)tiles, tmp, n_nl_d);
     CKR(cudaGetLastError());
     uint32_t n_nl = 0;
-    CKR(cudaMemcpyAsync(&n_nl, n_nl_d, 4, cudaMemcpyDeviceToHost, st));
-    CKR(cudaStreamSynchronize(st));
+    Readback rb(ctx);
+    CKR(rb.get(&n_nl, n_nl_d, 4));
+    CKR(rb.sync());
+    CKR(cudaEventElapsedTime(&copy_ms, ctx->ev[10], ctx->ev[11]));
     const uint64_t n_lines = n_nl + ((len > 0 && b[len - 1] != '\n') ? 1 : 0);
     uint64_t* nl;
     CKR(sc.get(&nl, std::max<uint64_t>(n_nl, 1)));
@@ -905,9 +962,9 @@ int upload_reads(swift_ctx* ctx, const char* b, size_t len, swift_reads** out,
     CKR(cudaGetLastError());
     unsigned long long h_err = 0;
     ParseSummary h_sum;
-    CKR(cudaMemcpyAsync(&h_err, err, sizeof(h_err), cudaMemcpyDeviceToHost, st));
-    CKR(cudaMemcpyAsync(&h_sum, sum, sizeof(h_sum), cudaMemcpyDeviceToHost, st));
-    CKR(cudaStreamSynchronize(st));
+    CKR(rb.get(&h_err, err, sizeof(h_err)));
+    CKR(rb.get(&h_sum, sum, sizeof(h_sum)));
+    CKR(rb.sync());
     if (h_err != ~0ull) {
       std::string m;
       const int code = parse_error((uint32_t)(h_err & 0xFF), h_err >> 8, &m, max_read);
@@ -921,7 +978,8 @@ int upload_reads(swift_ctx* ctx, const char* b, size_t len, swift_reads** out,
   }
 #undef CKR
   r->repeats = phase1_stale_repeats(r->n, r->n_gt);
-  if (parse_ms) *parse_ms = ms_since(t0);
+  if (h2d_ms) *h2d_ms = copy_ms;
+  if (parse_ms) *parse_ms = std::max(ms_since(t0) - copy_ms, 0.0);
   *out = r;
   return SWIFT_OK;
 }
@@ -964,6 +1022,7 @@ int swift_ctx_create(int device, void* stream, swift_ctx** out) {
     ctx->total_mem = (int64_t)tot;
   }
   for (int i = 0; i < kCtxEvents && e == cudaSuccess; ++i) e = cudaEventCreate(&ctx->ev[i]);
+  if (e == cudaSuccess) e = cudaMallocHost(&ctx->mail, kMailBytes);
   if (e != cudaSuccess) {
     delete ctx;
     return SWIFT_E_CUDA;
@@ -978,6 +1037,7 @@ int swift_ctx_destroy(swift_ctx* ctx) {
   cudaSetDevice(ctx->device);
   if (ctx->st) cudaStreamSynchronize(ctx->st);
   if (ctx->d_text) cudaFree(ctx->d_text);
+  if (ctx->mail) cudaFreeHost(ctx->mail);
   for (int i = 0; i < kCtxEvents; ++i)
     if (ctx->ev[i]) cudaEventDestroy(ctx->ev[i]);
   if (ctx->side) {
@@ -1555,8 +1615,9 @@ int swift_sw_pairs(swift_ctx* ctx, const char* qry, const int64_t* q_off, const 
   launch_var_max_len(st, dql, drl, n, mx);
   CKLAUNCH();
   int32_t h_mx[8];
-  CK(cudaMemcpyAsync(h_mx, mx, sizeof(h_mx), cudaMemcpyDeviceToHost, st));
-  CK(cudaStreamSynchronize(st));
+  Readback rb(ctx);
+  CK(rb.get(h_mx, mx, sizeof(h_mx)));
+  CK(rb.sync());
   const int maxQ = h_mx[0], maxR = h_mx[1];
   const int64_t n_long = h_mx[6];
   if (h_mx[2] < 1) return fail(ctx, SWIFT_E_ARG, "pair lengths must be >= 1");
@@ -1688,8 +1749,8 @@ int swift_sw_pairs(swift_ctx* ctx, const char* qry, const int64_t* q_off, const 
       CKLAUNCH();
       launches += k + 3;
       uint32_t nseg = 0;
-      CK(cudaMemcpyAsync(&nseg, nseg_d, 4, cudaMemcpyDeviceToHost, st));
-      CK(cudaStreamSynchronize(st));
+      CK(rb.get(&nseg, nseg_d, 4));
+      CK(rb.sync());
       std::vector<int32_t> hk(nseg), hs(nseg), hc(nseg);
       if (nseg) {
         CK(cudaMemcpyAsync(hk.data(), seg_key, nseg * 4, cudaMemcpyDeviceToHost, st));
@@ -2336,6 +2397,7 @@ static int align_resident_impl(swift_ctx* ctx, const swift_index* idx, const swi
     return SWIFT_OK;
   };
   int32_t h_cnt[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  Readback rb(ctx);
   int64_t pruned = 0;
   // list[0, *count) -> out in early-stop order (grid sized by max_n)
   int32_t *keys = nullptr, *sorted = nullptr;
@@ -2366,8 +2428,8 @@ static int align_resident_impl(swift_ctx* ctx, const swift_index* idx, const swi
     // scores it as well)
     CK(cudaEventRecord(ctx->ev[6], st));
     if (fast_ok && nproc > 0) {
-      CK(cudaMemcpyAsync(h_cnt, cnt, sizeof(h_cnt), cudaMemcpyDeviceToHost, st));
-      CK(cudaStreamSynchronize(st));
+      CK(rb.get(h_cnt, cnt, sizeof(h_cnt)));
+      CK(rb.sync());
       int32_t* sam_list = fast_list;
       if (lsuf) {
         // suffix LCS values for the early stop, then the order that groups
@@ -2398,8 +2460,8 @@ static int align_resident_impl(swift_ctx* ctx, const swift_index* idx, const swi
     launch_candidates(st, fa, tb_list, cnt + 2);
     CKLAUNCH();
     ++launches;
-    CK(cudaMemcpyAsync(h_cnt, cnt, sizeof(h_cnt), cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
+    CK(rb.get(h_cnt, cnt, sizeof(h_cnt)));
+    CK(rb.sync());
     CK(cudaEventRecord(ctx->ev[6], st));
     cand_n = h_cnt[2];
     fa2.cells_done = d_cells + 1;
@@ -2419,8 +2481,8 @@ static int align_resident_impl(swift_ctx* ctx, const swift_index* idx, const swi
     launch_prune(st, fa, aln, k1_list, cnt + 3);
     CKLAUNCH();
     ++launches;
-    CK(cudaMemcpyAsync(h_cnt, cnt, sizeof(h_cnt), cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
+    CK(rb.get(h_cnt, cnt, sizeof(h_cnt)));
+    CK(rb.sync());
     lcs_kept = h_cnt[3];
     if (lcs_kept > 0) {
       int32_t* ex_list = k1_list;
@@ -2451,8 +2513,8 @@ static int align_resident_impl(swift_ctx* ctx, const swift_index* idx, const swi
         pairs, keep, cand, nproc, fast_ok ? 0 : 1, list2, cnt + 4, cnt + 5);
     CKLAUNCH();
     ++launches;
-    CK(cudaMemcpyAsync(h_cnt, cnt, sizeof(h_cnt), cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
+    CK(rb.get(h_cnt, cnt, sizeof(h_cnt)));
+    CK(rb.sync());
     rc = trace_list(list2, cnt + 4, h_cnt[4], false);
     if (rc != SWIFT_OK) return rc;
     if (bounded) pruned = std::max<int64_t>(h_cnt[0] - h_cnt[2] - lcs_kept, 0);
@@ -2466,11 +2528,10 @@ static int align_resident_impl(swift_ctx* ctx, const swift_index* idx, const swi
   int scan_k = exclusive_scan_u64(st, bytes, offs, nproc, tmp, tot_d);
   CKLAUNCH();
   uint64_t total = 0;
-  CK(cudaMemcpyAsync(&total, tot_d, 8, cudaMemcpyDeviceToHost, st));
-  CK(cudaMemcpyAsync(h_cnt, cnt, sizeof(h_cnt), cudaMemcpyDeviceToHost, st));
+  CK(rb.get(&total, tot_d, 8));
+  CK(rb.get(h_cnt, cnt, sizeof(h_cnt)));
   unsigned long long h_cells2[2] = {0, 0}, h_model[kSeedModelSlots] = {};
-  CK(cudaMemcpyAsync(h_cells2, d_cells, sizeof(h_cells2), cudaMemcpyDeviceToHost, st));
-  const unsigned long long h_cells = h_cells2[0] + h_cells2[1];
+  CK(rb.get(h_cells2, d_cells, sizeof(h_cells2)));
   // a wave: each request's text starts at its first record's offset
   std::vector<uint64_t> h_t0;
   if (wave) {
@@ -2488,14 +2549,15 @@ static int align_resident_impl(swift_ctx* ctx, const swift_index* idx, const swi
     CKLAUNCH();
     ++launches;
     h_t0.resize(W + 1);
-    CK(cudaMemcpyAsync(h_t0.data(), d_t0, (W + 1) * 8, cudaMemcpyDeviceToHost, st));
+    CK(rb.get(h_t0.data(), d_t0, (W + 1) * 8));
   }
   if (so.d_model)
-    CK(cudaMemcpyAsync(h_model, so.d_model, sizeof(h_model), cudaMemcpyDeviceToHost, st));
+    CK(rb.get(h_model, so.d_model, sizeof(h_model)));
   TextChunks chunks;
-  rc = chunks.plan(ctx, st, offs, nproc, host_out != nullptr);
+  rc = chunks.plan(ctx, rb, offs, nproc, host_out != nullptr);
   if (rc != SWIFT_OK) return rc;
-  CK(cudaStreamSynchronize(st));
+  CK(rb.sync());
+  const unsigned long long h_cells = h_cells2[0] + h_cells2[1];
   if (wave)
     for (size_t r = 0; r < wave->size(); ++r) {
       (*wave)[r].text0 = h_t0[r];
@@ -3074,11 +3136,12 @@ static int align_paired_impl(swift_ctx* ctx, const swift_index* idx, const char*
   CKLAUNCH();
   launches += (covered > 0 ? 1 : 0) + exclusive_scan_u64(st, bytes, offs, (int64_t)covered, tmp2, tot2);
   uint64_t total = 0;
-  CK(cudaMemcpyAsync(&total, tot2, 8, cudaMemcpyDeviceToHost, st));
+  Readback rb(ctx);
+  CK(rb.get(&total, tot2, 8));
   TextChunks chunks;
-  rc = chunks.plan(ctx, st, offs, (int64_t)covered, host_out != nullptr);
+  rc = chunks.plan(ctx, rb, offs, (int64_t)covered, host_out != nullptr);
   if (rc != SWIFT_OK) return rc;
-  CK(cudaStreamSynchronize(st));
+  CK(rb.sync());
   char* d_text;
   CK(sc.get(&d_text, (size_t)total + 16));
   rc = chunks.write(ctx, st, fa, sam, d_text, total, host_out, host_cap, ctx->ev[5]);

@@ -12,6 +12,7 @@
 #include "internal.h"
 
 constexpr int kCtxEvents = 12;
+constexpr size_t kMailBytes = 16384;
 
 struct swift_ctx {
   int device = 0;
@@ -23,6 +24,8 @@ struct swift_ctx {
   char* d_text = nullptr;
   size_t text_len = 0, text_cap = 0;
   int sw_path = 0;  // 0 bounded selection, 1 generic kernel only, 2 exact score of every pair
+  // pinned landing place of the small copies the host waits for (Readback)
+  char* mail = nullptr;
   cudaStream_t side = nullptr;  // second stream for concurrent launches, made on first use
   cudaEvent_t fork_ev = nullptr, join_ev = nullptr;
   std::vector<cudaEvent_t> chunk_ev;  // per-chunk timing of the trace pass, grown on use

@@ -89,16 +89,18 @@ typedef struct {
   int64_t seed_overflow_strands, sw_generic_pairs;
   int64_t launches;   /* kernels this library launched for the call       */
   double host_parse_ms, h2d_ms, d2h_ms;  /* swift_align only: host side    */
-  int64_t traced_pairs;  /* pairs that went through the traceback pass       */
+  int64_t traced_pairs;  /* pairs whose alignment was traced: by the traceback
+                            pass, or along one diagonal by the gapless pass
+                            (there the printed ones)                         */
   int64_t bound_pruned;  /* pairs whose score bound ruled them out, so they
                             needed no exact score                            */
   int64_t retraced_pairs;/* printed pairs traced after selection (bounded
                             selection: the read's candidate was not best)    */
   double first_pass_ms;  /* the packed path's first kernel alone: the LCS
-                            bound (default) or the exact score pass; 0 with
-                            SAM output (every pair traced)                   */
+                            bound (default) or the exact score pass; 0 where
+                            every pair is traced (SAM output, small calls)   */
   int64_t first_pass_cells; /* DP cells that kernel covered               */
-  int64_t first_pass_kind;  /* 1 exact score, 3 LCS bound                 */
+  int64_t first_pass_kind;  /* 1 exact score, 3 LCS bound, 0 none         */
   double trace_ms;       /* trace-pass launches: the candidates (default;
                             they stop early on suffix LCS values) or every
                             packed pair over whole windows (SAM)            */

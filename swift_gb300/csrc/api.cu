@@ -401,6 +401,11 @@ __global__ void aln_to_ref_layout_kernel(const DevAln* __restrict__ aln, int64_t
   len[i] = a.len;
 }
 
+// With at most this many records left, tracing all of their pairs at once
+// costs less than the passes, lists and host round trips that would spare
+// most of them: at these sizes each pass lasts as long as one pair does.
+constexpr int64_t kDirectPairs = 3072;
+
 struct SeedOut {
   int32_t *m_read = nullptr, *m_strand = nullptr, *m_ri = nullptr, *m_sh = nullptr,
           *m_rp = nullptr;
@@ -2171,11 +2176,154 @@ static int align_resident_impl(swift_ctx* ctx, const swift_index* idx, const swi
       for (int64_t k = 0; k < q.nm; k += std::max<int64_t>(per, 1)) h_bs[q.rec0 + k] = 1;
     }
   }
+  // a wave of several query lengths: each read's own
+  uint8_t* d_bs = nullptr;
+  int32_t* d_rq = nullptr;
+  if (wave) {
+    CK(sc.get(&d_bs, (size_t)std::max<int64_t>(nm, 1)));
+    if (nm) CK(cudaMemcpyAsync(d_bs, h_bs.data(), nm, cudaMemcpyHostToDevice, st));
+    if (!uniform_q) {
+      std::vector<int32_t> h_rq((size_t)std::max<int64_t>(rd->n, 1), 0);
+      for (const WaveReq& q : *wave)
+        std::fill(h_rq.begin() + q.read0, h_rq.begin() + q.read0 + q.n, q.Q);
+      CK(sc.get(&d_rq, h_rq.size()));
+      CK(cudaMemcpyAsync(d_rq, h_rq.data(), h_rq.size() * 4, cudaMemcpyHostToDevice, st));
+    }
+  }
+  int bias = 0;
+  const bool fast_ok =
+      ctx->sw_path != 1 && fast_params_ok(Q, kWin, p->match, p->mismatch, p->gap_open, p->gap_ext, &bias);
+  // SAM output prints every record: no selection, every pair traced
+  const bool sam = p->out_format == 1;
+  const size_t nall = (size_t)std::max<int64_t>(nproc, 1);
+  const size_t nrd = (size_t)std::max<int64_t>(rd->n, 1);
+  int launches = 0;
+  // the reads' 2-bit queries and classes
+  ReadPackArgs rp;
+  memset(&rp, 0, sizeof(rp));
+  rp.reads = rd->d_bytes;
+  rp.rd = rd->d_rd;
+  rp.n_reads = rd->n;
+  rp.Q = Q;
+  rp.read_q = d_rq;
+  rp.words = code_words(Q);
+  CK(sc.get(&rp.read_cls, nrd));
+  CK(sc.get(&rp.codes, nrd * 2 * rp.words));
+  launch_pack_reads(st, rp);
+  CKLAUNCH();
+  launches += rd->n > 0 ? 1 : 0;
+  // Gapless pass: settles the reads with an alignment no gapped one can
+  // reach (with SAM output: the records); the rest go on below, all of it
+  // sized by their number.  `all`: the output's view of every record.
+  const int max_mis = gapless_max_mismatches(p->match, p->mismatch, p->gap_open, p->gap_ext);
+  // (a read's alignment starts about kShiftBases into its window: when the
+  // shortest query does not fit behind that, the pass settles next to none)
+  int min_q = Q;
+  if (wave)
+    for (const WaveReq& q : *wave) min_q = std::min(min_q, (int)q.Q);
+  const bool gapless = fast_ok && ctx->sw_path == 0 && max_mis >= 0 && idx->d_odd && nproc > 0 &&
+                       min_q <= kWin - kShiftBases + max_mis;
+  FormatArgs all;
+  memset(&all, 0, sizeof(all));
+  all.reads = rd->d_bytes;
+  all.rd = rd->d_rd;
+  all.recs = idx->d_recs;
+  all.cat = (const char*)idx->d_cat;
+  all.Q = Q;
+  all.read_q = d_rq;
+  all.n = nproc;
+  all.batch = per_iter > 0 ? per_iter : 1;
+  all.batch_start = d_bs;
+  LeftArgs left;
+  memset(&left, 0, sizeof(left));
+  left.m_read = so.m_read;
+  left.m_strand = so.m_strand;
+  left.m_ri = so.m_ri;
+  left.m_rp = so.m_rp;
+  left.n = nproc;
+  DevAln* all_aln = nullptr;
+  int64_t n = nproc;          // records left
+  int32_t settled[2] = {0, 0};  // records of settled groups, printed ones
+  if (gapless) {
+    GaplessArgs ga;
+    memset(&ga, 0, sizeof(ga));
+    ga.codes = rp.codes;
+    ga.read_cls = rp.read_cls;
+    ga.words = rp.words;
+    ga.ref = idx->d_packed;
+    ga.ref_words = (int64_t)((idx->cat_len + 15) / 16) + 2;
+    ga.odd = idx->d_odd;
+    ga.recs = idx->d_recs;
+    ga.m_read = so.m_read;
+    ga.m_strand = so.m_strand;
+    ga.m_ri = so.m_ri;
+    ga.m_rp = so.m_rp;
+    ga.n = nproc;
+    ga.Q = Q;
+    ga.read_q = d_rq;
+    ga.R = kWin;
+    ga.back = kShiftBases;
+    ga.match = p->match;
+    ga.mismatch = p->mismatch;
+    ga.gap_open = p->gap_open;
+    ga.max_mis = max_mis;
+    uint32_t *open, *at, *n_left;
+    int32_t* n_settled;
+    uint8_t* group_start;
+    void* tmp0;
+    CK(sc.get(&ga.pairs, nall));
+    CK(sc.get(&ga.aln, nall));
+    CK(sc.get(&ga.state, nall));
+    CK(sc.get(&all.keep, nall));
+    CK(sc.get(&open, nall));
+    CK(sc.get(&at, nall));
+    CK(sc.get(&group_start, nall));
+    CK(sc.get(&n_settled, 3));
+    CK(sc.get((uint8_t**)&tmp0, scan_temp_bytes(nproc)));
+    CK(cudaMemsetAsync(n_settled, 0, 3 * sizeof(int32_t), st));
+    n_left = (uint32_t*)(n_settled + 2);
+    launch_gapless(st, ga);
+    CKLAUNCH();
+    all.pairs = ga.pairs;
+    all.aln = all_aln = ga.aln;
+    if (sam)
+      launch_open(st, ga.state, nproc, open);
+    else
+      launch_settle(st, all, ga.state, open, group_start, n_settled);
+    CKLAUNCH();
+    launches += 2 + exclusive_scan_u32(st, open, at, nproc, tmp0, n_left);
+    int32_t h[3];
+    Readback rg(ctx);
+    CK(rg.get(h, n_settled, sizeof(h)));
+    CK(rg.sync());
+    n = h[2];
+    settled[0] = sam ? (int32_t)(nproc - n) : h[0];
+    settled[1] = h[1];
+    all.src = at;
+    const size_t nl = (size_t)std::max<int64_t>(n, 1);
+    left.open = open;
+    left.at = at;
+    left.group_start = sam ? nullptr : group_start;
+    CK(sc.get(&left.l_read, nl));
+    CK(sc.get(&left.l_strand, nl));
+    CK(sc.get(&left.l_ri, nl));
+    CK(sc.get(&left.l_rp, nl));
+    CK(sc.get(&left.l_of, nl));
+    CK(sc.get(&left.l_start, nl));
+    if (n > 0) {
+      launch_left(st, left);
+      CKLAUNCH();
+      ++launches;
+    }
+  }
+  // few records: each traced at once (see kDirectPairs); else bounded selection
+  const bool direct = fast_ok && ctx->sw_path == 0 && !sam && n <= kDirectPairs;
+  const bool bounded = fast_ok && ctx->sw_path == 0 && !sam && !direct;
   const int Qs = (Q + 16) & ~15;
   // consensus stride: Q + R + 2 bytes, rounded to 16 so the walk kernel can
   // store 32-bit words
   const int64_t cs = ((int64_t)Q + kWin + 2 + 15) & ~(int64_t)15;
-  const size_t nn = (size_t)std::max<int64_t>(nproc, 1);
+  const size_t nn = (size_t)std::max<int64_t>(n, 1);
   DevPair* pairs;
   char *qbuf, *wbuf, *qcons, *rcons;
   DevAln* aln;
@@ -2189,8 +2337,8 @@ static int align_resident_impl(swift_ctx* ctx, const swift_index* idx, const swi
   CK(sc.get(&qcons, nn * cs));
   CK(sc.get(&rcons, nn * cs));
   CK(sc.get(&keep, nn));
-  CK(sc.get(&bytes, nn));
-  CK(sc.get(&offs, nn));
+  CK(sc.get(&bytes, nall));
+  CK(sc.get(&offs, nall));
   CK(sc.get(&tot_d, 1));
   CK(sc.get((uint8_t**)&tmp, scan_temp_bytes(nproc)));
   PairArgs pa;
@@ -2202,50 +2350,30 @@ static int align_resident_impl(swift_ctx* ctx, const swift_index* idx, const swi
   pa.recs = idx->d_recs;
   pa.reads = rd->d_bytes;
   pa.rd = rd->d_rd;
-  pa.m_read = so.m_read;
-  pa.m_strand = so.m_strand;
-  pa.m_ri = so.m_ri;
-  pa.m_rp = so.m_rp;
-  pa.n = nproc;
+  pa.m_read = gapless ? left.l_read : so.m_read;
+  pa.m_strand = gapless ? left.l_strand : so.m_strand;
+  pa.m_ri = gapless ? left.l_ri : so.m_ri;
+  pa.m_rp = gapless ? left.l_rp : so.m_rp;
+  pa.n = n;
   pa.Q = Q;
   pa.pairs = pairs;
   pa.qbuf = qbuf;
   pa.wbuf = wbuf;
   pa.Qs = Qs;
-  uint8_t* read_cls;
-  CK(sc.get(&read_cls, (size_t)std::max<int64_t>(rd->n, 1)));
-  pa.read_cls = read_cls;
-  pa.n_reads = rd->n;
-  // a wave of several query lengths: each record's own, for the pair
-  // builder and every Smith-Waterman pass (rows past it match nothing)
+  pa.read_cls = rp.read_cls;
+  // each record's own query length, for the pair builder and every
+  // Smith-Waterman pass (rows past it match nothing)
   int32_t* pair_q = nullptr;
-  uint8_t* d_bs = nullptr;
-  if (wave) {
-    CK(sc.get(&d_bs, nn));
-    if (nm) CK(cudaMemcpyAsync(d_bs, h_bs.data(), nm, cudaMemcpyHostToDevice, st));
-    if (!uniform_q) {
-      std::vector<int32_t> h_rq((size_t)std::max<int64_t>(rd->n, 1), 0);
-      for (const WaveReq& q : *wave)
-        std::fill(h_rq.begin() + q.read0, h_rq.begin() + q.read0 + q.n, q.Q);
-      int32_t* d_rq;
-      CK(sc.get(&d_rq, h_rq.size()));
-      CK(cudaMemcpyAsync(d_rq, h_rq.data(), h_rq.size() * 4, cudaMemcpyHostToDevice, st));
-      CK(sc.get(&pair_q, nn));
-      pa.read_q = d_rq;
-      pa.pair_q = pair_q;
-    }
+  if (d_rq) {
+    CK(sc.get(&pair_q, nn));
+    pa.read_q = d_rq;
+    pa.pair_q = pair_q;
   }
   launch_build_pairs(st, pa);
   CKLAUNCH();
   CK(cudaEventRecord(ctx->ev[2], st));
   // split: packed score pass (then traceback of the printed pairs) or the
   // generic kernel (full result at once)
-  int bias = 0;
-  const bool fast_ok =
-      ctx->sw_path != 1 && fast_params_ok(Q, kWin, p->match, p->mismatch, p->gap_open, p->gap_ext, &bias);
-  // SAM output prints every record: no selection, every pair traced
-  const bool sam = p->out_format == 1;
-  const bool bounded = fast_ok && ctx->sw_path == 0 && !sam;
   // counters: 0 packed-path pairs, 1 generic pairs, 2 trace list,
   // 3 pairs the LCS bound keeps (exact-score list), 4 second trace list,
   // 5 printed records
@@ -2256,10 +2384,9 @@ static int align_resident_impl(swift_ctx* ctx, const swift_index* idx, const swi
   CK(sc.get(&tb_list, nn));
   CK(sc.get(&cnt, 8 + 4 * (kSufBlocks + 1)));
   CK(cudaMemsetAsync(cnt, 0, (8 + 4 * (kSufBlocks + 1)) * sizeof(int32_t), st));
-  int launches = 0;
-  if (nproc > 0) {
-    partition_pairs_kernel<<<(unsigned)((nproc + 255) / 256), 256, 0, st>>>(
-        pairs, nproc, fast_ok ? 0 : 1, fast_list, cnt, gen_list, cnt + 1);
+  if (n > 0) {
+    partition_pairs_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(
+        pairs, n, fast_ok ? 0 : 1, fast_list, cnt, gen_list, cnt + 1);
     CKLAUNCH();
     ++launches;
   }
@@ -2275,7 +2402,7 @@ static int align_resident_impl(swift_ctx* ctx, const swift_index* idx, const swi
   sa.mismatch = p->mismatch;
   sa.gap_open = p->gap_open;
   sa.gap_ext = p->gap_ext;
-  sa.n = nproc;
+  sa.n = n;
   sa.aln = aln;
   sa.qcons = qcons;
   sa.rcons = rcons;
@@ -2303,7 +2430,7 @@ static int align_resident_impl(swift_ctx* ctx, const swift_index* idx, const swi
   // suffix LCS values: early stop of the score and trace passes (bounded
   // selection; every pair traced with SAM output)
   uint16_t* lsuf = nullptr;
-  const bool lcs_stop = fast_ok && ctx->sw_path == 0;
+  const bool lcs_stop = fast_ok && ctx->sw_path == 0 && !direct;
   if (bounded) CK(sc.get(&cand, nn));
   if (lcs_stop) {
     CK(sc.get(&ub, nn));
@@ -2318,19 +2445,19 @@ static int align_resident_impl(swift_ctx* ctx, const swift_index* idx, const swi
   CK(cudaMemsetAsync(d_cells, 0, 2 * sizeof(unsigned long long), st));
   fa2.cells_done = d_cells;
   CK(cudaEventRecord(ctx->ev[7], st));
-  if (fast_ok && nproc > 0 && !sam) {
+  if (fast_ok && n > 0 && !sam && !direct) {
     fa2.list = fast_list;
     fa2.count = cnt;
     // bounded: the LCS bound of every packed pair, with its suffix values
     // (the exact pass runs later on the pairs it cannot rule out); else
     // exact scores
-    const int k = bounded ? launch_sw_lcs(st, fa2, nproc) : launch_sw_score(st, fa2, nproc);
+    const int k = bounded ? launch_sw_lcs(st, fa2, n) : launch_sw_score(st, fa2, n);
     if (k == 0) return fail(ctx, SWIFT_E_DEVICE, "first Smith-Waterman pass could not launch");
     launches += k;
     CKLAUNCH();
   }
   CK(cudaEventRecord(ctx->ev[8], st));
-  if (nproc > 0) {
+  if (n > 0) {
     sa.list = gen_list;
     sa.count = cnt + 1;
     rc = launch_sw(st, sa, &ctx->err);
@@ -2339,26 +2466,23 @@ static int align_resident_impl(swift_ctx* ctx, const swift_index* idx, const swi
     ++launches;
   }
   CK(cudaEventRecord(ctx->ev[3], st));
-  FormatArgs fa;
-  memset(&fa, 0, sizeof(fa));
-  fa.reads = rd->d_bytes;
-  fa.rd = rd->d_rd;
-  fa.recs = idx->d_recs;
+  FormatArgs fa = all;
+  fa.src = nullptr;
   fa.pairs = pairs;
   fa.aln = aln;
   fa.qcons = qcons;
   fa.rcons = rcons;
   fa.cons_stride = cs;
-  fa.n = nproc;
-  fa.batch = per_iter > 0 ? per_iter : 1;
-  fa.batch_start = d_bs;
+  fa.n = n;
+  // the records left keep the groups they had among all of them
+  if (gapless) fa.batch_start = left.l_start;
   fa.keep = keep;
   fa.bytes = bytes;
   fa.offs = offs;
   fa.ub = ub;
   fa.cand = cand;
   int2* best2 = nullptr;
-  if (fast_ok && nproc > 0) CK(sc.get(&best2, nn));
+  if (fast_ok && n > 0) CK(sc.get(&best2, nn));
   fa2.best = best2;
   // trace pass + walk over list[0, n), in chunks that bound the direction
   // scratch; `timed`: CUDA events around each chunk's trace pass
@@ -2427,7 +2551,7 @@ static int align_resident_impl(swift_ctx* ctx, const swift_index* idx, const swi
     // every record is printed: trace every packed-path pair (the trace pass
     // scores it as well)
     CK(cudaEventRecord(ctx->ev[6], st));
-    if (fast_ok && nproc > 0) {
+    if (fast_ok && n > 0) {
       CK(rb.get(h_cnt, cnt, sizeof(h_cnt)));
       CK(rb.sync());
       int32_t* sam_list = fast_list;
@@ -2452,8 +2576,13 @@ static int align_resident_impl(swift_ctx* ctx, const swift_index* idx, const swi
       fa2.lsuf = nullptr;
     }
   }
+  if (direct && n > 0) {
+    CK(cudaEventRecord(ctx->ev[6], st));
+    rc = trace_list(fast_list, cnt, n, false);
+    if (rc != SWIFT_OK) return rc;
+  }
   int64_t lcs_kept = 0, cand_n = 0;
-  if (bounded && nproc > 0) {
+  if (bounded && n > 0) {
     // candidates (largest LCS bound of their group) traced first; they stop
     // early on the LCS pass's suffix values, in an order that groups pairs
     // stopping alike
@@ -2503,21 +2632,37 @@ static int align_resident_impl(swift_ctx* ctx, const swift_index* idx, const swi
   if (!sam) {
     launch_select(st, fa);
     CKLAUNCH();
-    launches += nproc > 0 ? 1 : 0;
+    launches += n > 0 ? 1 : 0;
   }
-  if (!bounded && !sam) CK(cudaEventRecord(ctx->ev[6], st));
-  if (nproc > 0 && !sam) {
+  if ((!(bounded || direct) || n == 0) && !sam) CK(cudaEventRecord(ctx->ev[6], st));
+  if (n > 0 && !sam) {
     // printed packed-path pairs not traced yet
     int32_t* list2 = bounded ? gen_list : tb_list;  // generic list no longer needed
-    traceback_list_kernel<<<(unsigned)((nproc + 255) / 256), 256, 0, st>>>(
-        pairs, keep, cand, nproc, fast_ok ? 0 : 1, list2, cnt + 4, cnt + 5);
+    traceback_list_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(
+        pairs, keep, cand, n, fast_ok && !direct ? 0 : 1, list2, cnt + 4, cnt + 5);
     CKLAUNCH();
     ++launches;
-    CK(rb.get(h_cnt, cnt, sizeof(h_cnt)));
-    CK(rb.sync());
-    rc = trace_list(list2, cnt + 4, h_cnt[4], false);
-    if (rc != SWIFT_OK) return rc;
+    if (!direct) {
+      CK(rb.get(h_cnt, cnt, sizeof(h_cnt)));
+      CK(rb.sync());
+      rc = trace_list(list2, cnt + 4, h_cnt[4], false);
+      if (rc != SWIFT_OK) return rc;
+    }
     if (bounded) pruned = std::max<int64_t>(h_cnt[0] - h_cnt[2] - lcs_kept, 0);
+  }
+  if (gapless) {
+    // back among all records, whose text is written from here on
+    if (n > 0) {
+      launch_put_back(st, left.l_of, aln, keep, n, all_aln, sam ? nullptr : all.keep);
+      CKLAUNCH();
+      ++launches;
+    }
+    all.qcons = qcons;
+    all.rcons = rcons;
+    all.cons_stride = cs;
+    all.bytes = bytes;
+    all.offs = offs;
+    fa = all;
   }
   CK(cudaEventRecord(ctx->ev[4], st));
   if (sam)
@@ -2595,8 +2740,8 @@ static int align_resident_impl(swift_ctx* ctx, const swift_index* idx, const swi
     if (!sam) {
       cudaEventElapsedTime(&t, ctx->ev[7], ctx->ev[8]);
       s.first_pass_ms = t;
-      s.first_pass_kind = bounded ? 3 : 1;
-      s.first_pass_cells = fast_ok ? (int64_t)h_cnt[0] * Q * kWin : 0;
+      s.first_pass_kind = direct ? 0 : bounded ? 3 : 1;
+      s.first_pass_cells = fast_ok && !direct ? (int64_t)h_cnt[0] * Q * kWin : 0;
     }
     s.lcs_kept = lcs_kept;
     s.seed_kernel_ms = so.kernel_ms;
@@ -2617,14 +2762,14 @@ static int align_resident_impl(swift_ctx* ctx, const swift_index* idx, const swi
     s.cells = nproc * (int64_t)Q * kWin;
     s.out_bytes = (int64_t)total;
     s.seed_overflow_strands = so.overflow;
-    s.printed = sam ? nproc : h_cnt[5];
+    s.printed = sam ? nproc : h_cnt[5] + settled[1];
     s.sw_generic_pairs = h_cnt[1];
-    s.traced_pairs = sam ? h_cnt[0] : h_cnt[2] + h_cnt[4];
-    s.bound_pruned = pruned;
+    s.traced_pairs = sam ? h_cnt[0] + settled[0] : (direct ? h_cnt[0] : h_cnt[2] + h_cnt[4]) + settled[1];
+    s.bound_pruned = pruned + (sam ? 0 : settled[0] - settled[1]);
     s.retraced_pairs = bounded ? h_cnt[4] : 0;
     // build_pairs + the Smith-Waterman passes and select (launches) +
     // format sizes, scan, format write (one per record range)
-    s.launches = so.launches + (nproc > 0 ? 1 + 1 + chunks.n_chunks : 0) + launches + scan_k;
+    s.launches = so.launches + (n > 0 ? 1 : 0) + (nproc > 0 ? 1 + chunks.n_chunks : 0) + launches + scan_k;
     *stats = s;
   }
   return SWIFT_OK;

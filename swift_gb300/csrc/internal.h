@@ -110,8 +110,12 @@ struct DevPair {
   int32_t ref_idx;
   int32_t ref_dist;       // max(0, refPos - 100)
   int32_t win_len;        // window bases after N trimming
-  int32_t flags;          // bit 0: needs the generic SW kernel
+  int32_t flags;          // bit 0: needs the generic SW kernel; kPairGapless
 };
+// Set by the gapless pass (ungapped.cu) on the records it settled: no window
+// or query bytes were written out for them, the strings are read in place,
+// and win_len holds the alignment's first query row (from 0).
+constexpr int32_t kPairGapless = 2;
 
 // Result of one Smith-Waterman pair.
 struct DevAln {
@@ -313,11 +317,74 @@ struct PairArgs {
   char* qbuf;                 // n x Qs
   char* wbuf;                 // n x kWinPad
   int Qs;                     // query stride (>= every query length + 1)
-  uint8_t* read_cls;          // optional scratch, n_reads bytes: per read 0 when its
-                              // query bytes are all A, C, G or T (word-wise copy)
-  int64_t n_reads;
+  const uint8_t* read_cls;    // optional (launch_pack_reads): per read 0 when its query
+                              // bytes are all A, C, G or T (word-wise copy)
 };
 void launch_build_pairs(cudaStream_t st, const PairArgs& a);
+
+// ungapped.cu: 2-bit codes of the reads' queries, and the gapless pass
+constexpr int kReadCodeWords = kMaxQ / 16;
+inline int code_words(int Q) { return (Q + 15) / 16; }
+struct ReadPackArgs {
+  const char* reads;
+  const DevRead* rd;
+  int64_t n_reads;
+  int Q;                      // query length, or the longest with read_q
+  const int32_t* read_q;      // optional: query length per read
+  int words;                  // code words per strand: code_words(Q)
+  uint8_t* read_cls;          // out, per read: 0 when its query is all A, C, G or T
+  uint32_t* codes;            // out, class 0 reads: [read][strand][words]
+};
+void launch_pack_reads(cudaStream_t st, const ReadPackArgs& a);
+enum : uint8_t {
+  kGaplessOther = 0,          // not looked at: its score can be anything
+  kGaplessBounded = 1,        // its score is at most match * Q + gap_open
+  kGaplessDone = 2,           // settled: aln holds its result, above that bound
+};
+constexpr int kGaplessMaxMis = 6;
+struct GaplessArgs {
+  const uint32_t* codes;      // of launch_pack_reads, with its read_cls and words
+  const uint8_t* read_cls;
+  int words;
+  const uint32_t* ref;        // 2-bit codes of the concatenated sequences
+  int64_t ref_words;
+  const uint32_t* odd;        // bit per base that is not ACGTacgt
+  const DevRecord* recs;
+  const int32_t* m_read;      // per record: read, strand, ref idx, ref pos
+  const int32_t* m_strand;
+  const int32_t* m_ri;
+  const int32_t* m_rp;
+  const int32_t* m_mate;      // optional: mate 2's reads start at mate2
+  int32_t mate2;
+  int64_t n;
+  int Q;
+  const int32_t* read_q;      // optional: query length per read
+  int R, back;                // window: R bases from max(0, ref pos - back)
+  int match, mismatch, gap_open;
+  int max_mis;                // gapless_max_mismatches(...)
+  DevPair* pairs;             // out
+  DevAln* aln;                // out: the settled records' results
+  uint8_t* state;             // out
+};
+// The mismatches a diagonal may hold and still beat every gapped alignment;
+// -1: the gapless pass does not take this scoring.  Above kGaplessMaxMis its
+// 16-row test would pass by chance too often (1 % of the diagonals at 7).
+int gapless_max_mismatches(int match, int mismatch, int gap_open, int gap_ext);
+void launch_gapless(cudaStream_t st, const GaplessArgs& a);
+// The records left to the Smith-Waterman passes, in order: open[j] != 0 (a
+// scan of it in at[j]) are copied to m_*[at[j]] with their index and, when
+// group_start is given, its flag.
+struct LeftArgs {
+  int64_t n;
+  const uint32_t* open;
+  const uint32_t* at;
+  const int32_t *m_read, *m_strand, *m_ri, *m_rp;
+  const uint8_t* group_start; // optional
+  int32_t *l_read, *l_strand, *l_ri, *l_rp;
+  int32_t* l_of;              // out: their record
+  uint8_t* l_start;
+};
+void launch_left(cudaStream_t st, const LeftArgs& a);
 
 // paired.cu: *bad = 1 when a read name of either file does not end in 1 or 2
 void launch_pe_names(cudaStream_t st, const char* b1, const DevRead* rd1, const char* b2,
@@ -557,11 +624,28 @@ struct FormatArgs {
   char* text;
   const int32_t* ub;          // bounded selection: upper bound per packed-path pair
   int32_t* cand;              // bounded selection: the group's candidate per pair
+  // records settled by the gapless pass (kPairGapless) read their strings in
+  // place; the others' strings are at src[j] (null: at j)
+  const uint32_t* src;
+  const char* cat;            // concatenated sequences
+  int Q;                      // query length, or with read_q each read's
+  const int32_t* read_q;
   const int8_t* pe_sep;       // paired-end records (printOutput_paired2): 1 opens a
                               // pair with a line of 37 '*', 0 a blank line; null:
                               // the single-end record's 40 '*'
 };
 void launch_select(cudaStream_t st, const FormatArgs& a);
+// The best-per-read groups the gapless pass settles: keep is written for
+// them, open[j] = 1 for the records of the others (group_start[j] = 1 at
+// their first); n_settled counts the settled groups' records and printed ones.
+void launch_settle(cudaStream_t st, const FormatArgs& a, const uint8_t* state, uint32_t* open,
+                   uint8_t* group_start, int32_t* n_settled);
+// every record not settled by itself is open (no groups: SAM output)
+void launch_open(cudaStream_t st, const uint8_t* state, int64_t n, uint32_t* open);
+// results of the records left to the Smith-Waterman passes, back to their
+// places (keep and l_keep optional)
+void launch_put_back(cudaStream_t st, const int32_t* l_of, const DevAln* l_aln,
+                     const int32_t* l_keep, int64_t n, DevAln* aln, int32_t* keep);
 void launch_candidates(cudaStream_t st, const FormatArgs& a, int32_t* list, int32_t* cnt);
 void launch_prune(cudaStream_t st, const FormatArgs& a, DevAln* aln, int32_t* list, int32_t* cnt);
 void launch_format_sizes(cudaStream_t st, const FormatArgs& a);

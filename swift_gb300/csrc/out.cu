@@ -82,6 +82,91 @@ __global__ void select_kernel(FormatArgs a) {
   for (int64_t i = j; i <= e; ++i) a.keep[i] = i == keep ? 1 : 0;
 }
 
+// The groups the gapless pass (ungapped.cu) settles: it looked at every
+// record, and settled one at least.  Its unsettled records score at most its
+// bound, below every settled one, so the group's pick is its first largest
+// settled score.  The other groups are left open, whole.
+__global__ void settle_kernel(FormatArgs a, const uint8_t* __restrict__ state, uint32_t* open,
+                              uint8_t* group_start, int32_t* n_settled) {
+  const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  int settled = 0;
+  if (j < a.n && (opens_batch(a, j) || !names_equal(a, a.pairs[j], a.pairs[j - 1]))) {
+    const int64_t e = group_end(a, j);
+    int64_t pick = -1;
+    int mx = 0;
+    bool known = true;
+    for (int64_t i = j; i <= e; ++i) {
+      const uint8_t s = state[i];
+      known = known && s != kGaplessOther;
+      if (s == kGaplessDone && a.aln[i].score > mx) {
+        mx = a.aln[i].score;
+        pick = i;
+      }
+    }
+    if (!known) pick = -1;
+    for (int64_t i = j; i <= e; ++i) {
+      a.keep[i] = i == pick ? 1 : 0;
+      open[i] = pick < 0 ? 1u : 0u;
+      group_start[i] = i == j ? 1 : 0;
+    }
+    if (pick >= 0) settled = (int)(e - j + 1);
+  }
+  block_count(settled > 0, n_settled + 1);
+  settled = __reduce_add_sync(0xffffffffu, settled);
+  if ((threadIdx.x & 31) == 0 && settled) atomicAdd(n_settled, settled);
+}
+
+__global__ void open_kernel(const uint8_t* __restrict__ state, int64_t n, uint32_t* open) {
+  const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (j < n) open[j] = state[j] == kGaplessDone ? 0u : 1u;
+}
+
+__global__ void put_back_kernel(const int32_t* __restrict__ l_of, const DevAln* __restrict__ l_aln,
+                                const int32_t* __restrict__ l_keep, int64_t n, DevAln* aln,
+                                int32_t* keep) {
+  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= n) return;
+  const int32_t j = l_of[t];
+  aln[j] = l_aln[t];
+  if (keep) keep[j] = l_keep[t];
+}
+
+// The strings of a record's alignment, position z = 0, 1, ... in printing
+// order: read in place from the read and the concatenated sequences for a
+// record the gapless pass settled, else from the reversed consensus strings.
+struct AlnStrings {
+  const char *r, *q;
+  int step;    // of q
+  int r_step;  // of r
+  bool comp;   // complement the query's bases
+  __device__ __forceinline__ char ref(int z) const { return r[z * r_step]; }
+  __device__ __forceinline__ char qry(int z) const {
+    const char c = q[z * step];
+    if (!comp) return c;
+    return c == 'A' ? 'T' : c == 'C' ? 'G' : c == 'G' ? 'C' : 'A';
+  }
+};
+__device__ __forceinline__ AlnStrings aln_strings(const FormatArgs& a, int64_t j, const DevPair& p,
+                                                  const DevAln& al) {
+  AlnStrings s;
+  if (p.flags & kPairGapless) {
+    const int Q = a.read_q ? a.read_q[p.read] : a.Q;
+    const char* read = a.reads + a.rd[p.read].seq_off;
+    s.r = a.cat + a.recs[p.ref_idx].cat_start + p.ref_dist + (al.start - 1);
+    s.r_step = 1;
+    s.comp = p.strand != 0;
+    s.q = s.comp ? read + (Q - 1 - p.win_len) : read + p.win_len;
+    s.step = s.comp ? -1 : 1;
+  } else {
+    const int64_t at = (a.src ? (int64_t)a.src[j] : j) * a.cons_stride + (al.len - 1);
+    s.r = a.rcons + at;
+    s.q = a.qcons + at;
+    s.step = s.r_step = -1;
+    s.comp = false;
+  }
+  return s;
+}
+
 // Bounded selection, step 1: per best-per-read group (the groups of
 // select_kernel) the candidate is the first pair with the largest key, the
 // exact score for pairs of the generic kernel and the upper bound for the
@@ -264,11 +349,10 @@ __global__ void __launch_bounds__(kFmtWarps * 32) format_write_kernel(FormatArgs
     }
     char* out = q + 4;
     const int L = al.len > 0 ? al.len : 0;
-    const char* rc = a.rcons + j * a.cons_stride;
-    const char* qc = a.qcons + j * a.cons_stride;
-    // "R: " already written; reversed strings
+    const AlnStrings str = aln_strings(a, j, p, al);
+    // "R: " already written
     for (int z = lane; z < L; z += 32) {
-      const char r = rc[L - 1 - z], qq = qc[L - 1 - z];
+      const char r = str.ref(z), qq = str.qry(z);
       out[z] = r;
       const int ur = (unsigned)(r - 'a') < 26u ? r - 32 : r;
       const int uq = (unsigned)(qq - 'a') < 26u ? qq - 32 : qq;
@@ -319,7 +403,12 @@ __global__ void sam_sizes_kernel(FormatArgs a) {
   const DevAln al = a.aln[j];
   const int L = al.len > 0 ? al.len : 0;
   uint64_t n = qname_len(a, p) + 3 + a.recs[p.ref_idx].name_len + 1 + ndigits(al.start) + 5;
-  n += cigar_bytes(a.rcons + j * a.cons_stride, a.qcons + j * a.cons_stride, L);
+  if (p.flags & kPairGapless) {
+    n += ndigits(L) + 1;  // one run of M
+  } else {
+    const int64_t at = (a.src ? (int64_t)a.src[j] : j) * a.cons_stride;
+    n += cigar_bytes(a.rcons + at, a.qcons + at, L);
+  }
   n += 7 + L + 3;
   a.bytes[j] = n;
 }
@@ -342,14 +431,13 @@ __global__ void __launch_bounds__(kFmtWarps * 32) sam_write_kernel(FormatArgs a)
   const DevPair p = a.pairs[j];
   const DevAln al = a.aln[j];
   const int L = al.len > 0 ? al.len : 0;
-  const char* rc = a.rcons + j * a.cons_stride;
-  const char* qc = a.qcons + j * a.cons_stride;
+  const AlnStrings str = aln_strings(a, j, p, al);
   char* head = head_all[wib];
   char* ops = ops_all[wib];
   uint32_t* starts = starts_all[wib];
   // the operations in printing order (last consensus byte first), and a bit
   // per position that starts a run
-  for (int t = lane; t < L; t += 32) ops[t] = cigar_op(rc[L - 1 - t], qc[L - 1 - t]);
+  for (int t = lane; t < L; t += 32) ops[t] = cigar_op(str.ref(t), str.qry(t));
   __syncwarp();
   for (int c0 = 0; c0 < L; c0 += 32) {
     const int t = c0 + lane;
@@ -394,7 +482,7 @@ __global__ void __launch_bounds__(kFmtWarps * 32) sam_write_kernel(FormatArgs a)
   char* out = a.text + a.offs[j];
   for (int i = lane; i < hn; i += 32) out[i] = head[i];
   out += hn;
-  for (int z = lane; z < L; z += 32) out[z] = qc[L - 1 - z];
+  for (int z = lane; z < L; z += 32) out[z] = str.qry(z);
   if (lane == 0) {
     out[L] = '\t';
     out[L + 1] = '*';
@@ -418,6 +506,23 @@ void launch_sam_write(cudaStream_t st, const FormatArgs& a) {
 void launch_select(cudaStream_t st, const FormatArgs& a) {
   if (a.n <= 0) return;
   select_kernel<<<(unsigned)((a.n + 255) / 256), 256, 0, st>>>(a);
+}
+
+void launch_settle(cudaStream_t st, const FormatArgs& a, const uint8_t* state, uint32_t* open,
+                   uint8_t* group_start, int32_t* n_settled) {
+  if (a.n <= 0) return;
+  settle_kernel<<<(unsigned)((a.n + 255) / 256), 256, 0, st>>>(a, state, open, group_start, n_settled);
+}
+
+void launch_open(cudaStream_t st, const uint8_t* state, int64_t n, uint32_t* open) {
+  if (n <= 0) return;
+  open_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(state, n, open);
+}
+
+void launch_put_back(cudaStream_t st, const int32_t* l_of, const DevAln* l_aln,
+                     const int32_t* l_keep, int64_t n, DevAln* aln, int32_t* keep) {
+  if (n <= 0) return;
+  put_back_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(l_of, l_aln, l_keep, n, aln, keep);
 }
 
 void launch_candidates(cudaStream_t st, const FormatArgs& a, int32_t* list, int32_t* cnt) {

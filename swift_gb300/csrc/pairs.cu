@@ -42,32 +42,6 @@ __device__ __forceinline__ uint32_t comp4(uint32_t x) {
   return x ^ ((((~x) >> 1) & 0x01010101u) * 0x11u | 0x04040404u);
 }
 
-// Per read: 0 when its query (the first Q bytes, Q <= its length) is all
-// upper-case A, C, G, T, so that both strands' queries are whole-word
-// copies; else 1 (the per-byte path of build_pairs_kernel).
-constexpr int kClsRounds = 10;  // queries up to 320 bytes
-
-__global__ void read_class_kernel(PairArgs a) {
-  const int lane = threadIdx.x & 31;
-  const int64_t r = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (r >= a.n_reads) return;
-  const DevRead rd = a.rd[r];
-  const int Q = a.read_q ? a.read_q[r] : a.Q;
-  bool bad = rd.len < Q || Q > 32 * kClsRounds;
-  const char* s = a.reads + rd.seq_off;
-  if (!bad) {
-    // every byte loaded before any is tested
-    char c[kClsRounds];
-#pragma unroll
-    for (int t = 0; t < kClsRounds; ++t) c[t] = lane + 32 * t < Q ? s[lane + 32 * t] : 'A';
-#pragma unroll
-    for (int t = 0; t < kClsRounds; ++t)
-      bad |= !(c[t] == 'A' || c[t] == 'C' || c[t] == 'G' || c[t] == 'T');
-  }
-  bad = __any_sync(0xffffffffu, bad);
-  if (lane == 0) a.read_cls[r] = bad ? 1 : 0;
-}
-
 // getRefSeq2's walk over the file bytes: up to 300 characters from file
 // offset off, newlines dropped, stopping at a header line or end of file.
 // The first kPre 32-byte rounds are loaded up front so the warp waits for
@@ -279,8 +253,6 @@ __global__ void __launch_bounds__(kPairWarps * 32) build_pairs_kernel(PairArgs a
 
 void launch_build_pairs(cudaStream_t st, const PairArgs& a) {
   if (a.n <= 0) return;
-  if (a.read_cls && a.n_reads > 0)
-    read_class_kernel<<<(unsigned)((a.n_reads * 32 + 255) / 256), 256, 0, st>>>(a);
   unsigned grid = (unsigned)((a.n + kPairWarps - 1) / kPairWarps);
   build_pairs_kernel<<<grid, kPairWarps * 32, 0, st>>>(a);
 }

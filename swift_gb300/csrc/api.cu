@@ -2945,8 +2945,9 @@ static int align_paired_impl(swift_ctx* ctx, const swift_index* idx, const char*
     launch_pe_names(st, rd1->d_bytes, rd1->d_rd, rd2->d_bytes, rd2->d_rd, n, d_bad);
     CKLAUNCH();
     int32_t bad = 0;
-    CK(cudaMemcpyAsync(&bad, d_bad, sizeof(bad), cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
+    Readback rn(ctx);
+    CK(rn.get(&bad, d_bad, sizeof(bad)));
+    CK(rn.sync());
     if (bad) return fail(ctx, SWIFT_E_INPUT, "paired-end read names must end in 1 or 2");
   }
   rc = ensure_lt2(ctx, idx);
@@ -3010,13 +3011,11 @@ static int align_paired_impl(swift_ctx* ctx, const swift_index* idx, const char*
   CKLAUNCH();
   int launches = (int)so.launches + (n > 0 ? 1 : 0) + exclusive_scan_u64(st, cnt, roff, n, tmp, tot_d);
   uint64_t nrec = 0;
-  CK(cudaMemcpyAsync(&nrec, tot_d, 8, cudaMemcpyDeviceToHost, st));
-  std::vector<uint64_t> h_cnt((size_t)std::max<int64_t>(n, 1));
-  if (n) CK(cudaMemcpyAsync(h_cnt.data(), cnt, n * 8, cudaMemcpyDeviceToHost, st));
-  CK(cudaStreamSynchronize(st));
+  Readback rb(ctx);
+  CK(rb.get(&nrec, tot_d, 8));
+  CK(rb.sync());
   const size_t nr = (size_t)std::max<uint64_t>(nrec, 1);
   CK(sc.get(&pa.m_id, nr));
-  CK(sc.get(&pa.m_mate, nr));
   CK(sc.get(&pa.m_rev, nr));
   CK(sc.get(&pa.m_read, nr));
   CK(sc.get(&pa.m_ri, nr));
@@ -3038,153 +3037,28 @@ static int align_paired_impl(swift_ctx* ctx, const swift_index* idx, const char*
   if (n) CK(cudaMemcpyAsync(d_rd, rd1->d_rd, n * sizeof(DevRead), cudaMemcpyDeviceToDevice, st));
   launch_shift_reads(st, rd2->d_rd, n, len1, d_rd + n);
   CKLAUNCH();
-  // Phase 2 pairs: query Q, window 3Q; the packed passes trace pairs of
-  // ACGT bytes with full windows, the generic kernel the others
   const int R = 3 * Q;
-  const int64_t qs = (Q + 16) & ~15, ws = (R + 16) & ~15;
-  const int64_t cs = ((int64_t)Q + R + 2 + 15) & ~(int64_t)15;  // the walk stores words
-  char *qbuf, *wbuf, *qcons, *rcons;
-  DevPair* pairs;
-  DevAln* aln;
-  CK(sc.get(&qbuf, nr * qs));
-  CK(sc.get(&wbuf, nr * ws));
-  CK(sc.get(&qcons, nr * cs));
-  CK(sc.get(&rcons, nr * cs));
-  CK(sc.get(&pairs, nr));
-  CK(sc.get(&aln, nr));
-  CK(cudaMemsetAsync(wbuf, 0, nr * ws, st));
-  pa.Q = Q;
-  pa.ref_file = idx->d_file;
-  pa.cat = (const char*)idx->d_cat;
-  pa.odd = idx->d_odd;
-  pa.ref_file_len = idx->file_len;
-  pa.recs = idx->d_recs;
-  pa.reads = d_reads;
-  pa.rd = d_rd;
-  pa.pairs = pairs;
-  pa.qbuf = qbuf;
-  pa.wbuf = wbuf;
-  pa.q_stride = qs;
-  pa.w_stride = ws;
-  launch_pe_pairs(st, pa);
-  CKLAUNCH();
-  ++launches;
-  CK(cudaEventRecord(ctx->ev[2], st));
-  int bias = 0;
-  const bool fast_ok = fast_params_ok(Q, R, p->match, p->mismatch, p->gap_open, p->gap_ext, &bias);
-  int32_t *fast_list, *gen_list, *lcnt;
-  CK(sc.get(&fast_list, nr));
-  CK(sc.get(&gen_list, nr));
-  CK(sc.get(&lcnt, 2));
-  CK(cudaMemsetAsync(lcnt, 0, 2 * sizeof(int32_t), st));
-  if (nrec > 0) {
-    partition_pairs_kernel<<<(unsigned)((nrec + 255) / 256), 256, 0, st>>>(
-        pairs, (int64_t)nrec, fast_ok ? 0 : 1, fast_list, lcnt, gen_list, lcnt + 1);
-    CKLAUNCH();
-    ++launches;
-    SwArgs sa;
-    memset(&sa, 0, sizeof(sa));
-    sa.q = qbuf;
-    sa.w = wbuf;
-    sa.q_stride = qs;
-    sa.w_stride = ws;
-    sa.Q = Q;
-    sa.R = R;
-    sa.match = p->match;
-    sa.mismatch = p->mismatch;
-    sa.gap_open = p->gap_open;
-    sa.gap_ext = p->gap_ext;
-    sa.n = (int64_t)nrec;
-    sa.aln = aln;
-    sa.qcons = qcons;
-    sa.rcons = rcons;
-    sa.cons_stride = cs;
-    sa.list = gen_list;
-    sa.count = lcnt + 1;
-    rc = launch_sw(st, sa, &ctx->err);
-    if (rc != SWIFT_OK) return rc;
-    CKLAUNCH();
-    ++launches;
-    if (fast_ok) {
-      int32_t h_fast = 0;
-      CK(cudaMemcpyAsync(&h_fast, lcnt, 4, cudaMemcpyDeviceToHost, st));
-      CK(cudaStreamSynchronize(st));
-      const int64_t chunk = 262144;
-      int2* best2;
-      uint32_t* dirs;
-      CK(sc.get(&best2, nr));
-      CK(sc.get(&dirs, (size_t)trace_scratch_words(Q, R, std::min<int64_t>(std::max(h_fast, 1), chunk))));
-      FastArgs fa2;
-      memset(&fa2, 0, sizeof(fa2));
-      fa2.q = qbuf;
-      fa2.w = wbuf;
-      fa2.q_stride = qs;
-      fa2.w_stride = ws;
-      fa2.Q = Q;
-      fa2.R = R;
-      fa2.match = p->match;
-      fa2.mismatch = p->mismatch;
-      fa2.gap_open = p->gap_open;
-      fa2.gap_ext = p->gap_ext;
-      fa2.bias = bias;
-      fa2.aln = aln;
-      fa2.qcons = qcons;
-      fa2.rcons = rcons;
-      fa2.cons_stride = cs;
-      fa2.best = best2;
-      fa2.list = fast_list;
-      fa2.count = lcnt;
-      fa2.dirs = dirs;
-      for (int64_t off = 0; off < h_fast; off += chunk) {
-        fa2.list_offset = off;
-        const int kk = launch_sw_trace(st, fa2, std::min<int64_t>(chunk, h_fast - off));
-        if (kk == 0) return fail(ctx, SWIFT_E_DEVICE, "trace pass could not launch");
-        launches += kk;
-        CKLAUNCH();
-      }
-    }
-  }
-  CK(cudaEventRecord(ctx->ev[3], st));
-  // selection (chooseBestAlignment_paired3 per batch) on the host over the
-  // per-record scores, names and coordinates; printing flags to the device
-  const bool sam = p->out_format == 1;
-  FormatArgs fa;
-  memset(&fa, 0, sizeof(fa));
-  fa.reads = d_reads;
-  fa.rd = d_rd;
-  fa.recs = idx->d_recs;
-  fa.pairs = pairs;
-  fa.aln = aln;
-  fa.qcons = qcons;
-  fa.rcons = rcons;
-  fa.cons_stride = cs;
-  fa.n = (int64_t)nrec;
-  int32_t* keep;
-  int8_t* sep;
-  uint64_t *bytes, *offs, *tot2;
-  void* tmp2;
-  CK(sc.get(&keep, nr));
-  CK(sc.get(&sep, nr));
-  CK(sc.get(&bytes, nr));
-  CK(sc.get(&offs, nr));
-  CK(sc.get(&tot2, 1));
-  CK(sc.get((uint8_t**)&tmp2, scan_temp_bytes((int64_t)nrec)));
   // Phase-2 batches: getNumQueriesPerIteration_paired (src/align.cu:2804-2824)
   // and getNumQrsPerIter_paired (src/align.cu:1812-1852) over the record ids,
   // which follow from the per-pair record counts; records past the last
   // batch are not aligned in the reference and not printed here
-  std::vector<uint8_t> h_bs(nr, 0);
-  uint64_t covered = 0;
+  uint8_t* d_bs;
+  CK(sc.get(&d_bs, nr));
+  int64_t covered = 0;
   {
     const int64_t dev_mem = p->device_mem > 0 ? p->device_mem : ctx->total_mem;
-    int64_t max_per;
-    {
-      const int mem_pair = (R + 1) + (Q + 1) + 4 + 4 + 4 + 2 + 2 * (Q + R + 2);
-      const long gm = (long)(dev_mem - 100000000LL);
-      max_per = (int)floor((float)gm / mem_pair);
-      if (max_per > (int64_t)nrec) max_per = (int64_t)nrec;
-    }
-    if (max_per > 0) {
+    const int mem_pair = (R + 1) + (Q + 1) + 4 + 4 + 4 + 2 + 2 * (Q + R + 2);
+    const long gm = (long)(dev_mem - 100000000LL);
+    const int64_t max_per = (int)floor((float)gm / mem_pair);
+    if (nrec > 0 && max_per >= (int64_t)nrec) {
+      // one batch of all records
+      covered = (int64_t)nrec;
+      CK(cudaMemsetAsync(d_bs, 0, nr, st));
+      CK(cudaMemsetAsync(d_bs, 1, 1, st));
+    } else if (max_per > 0 && nrec > 0) {
+      std::vector<uint64_t> h_cnt((size_t)n);
+      CK(cudaMemcpyAsync(h_cnt.data(), cnt, n * 8, cudaMemcpyDeviceToHost, st));
+      CK(cudaStreamSynchronize(st));
       std::vector<int64_t> per;
       int64_t old_count = 0, count = 0, old_id = 0;
       bool is_new = false;
@@ -3207,15 +3081,68 @@ static int align_paired_impl(swift_ctx* ctx, const swift_index* idx, const char*
           old_id = id;
         }
       if (!is_new && count <= max_per) per.push_back(count);
+      std::vector<uint8_t> h_bs(nr, 0);
       for (int64_t c : per) {
-        if (covered < nrec) h_bs[covered] = 1;
-        covered += (uint64_t)c;
+        if (covered < (int64_t)nrec) h_bs[covered] = 1;
+        covered += c;
       }
-      covered = std::min<uint64_t>(covered, nrec);
+      covered = std::min<int64_t>(covered, (int64_t)nrec);
+      if (covered) CK(cudaMemcpyAsync(d_bs, h_bs.data(), covered, cudaMemcpyHostToDevice, st));
     }
   }
-  fa.n = (int64_t)covered;
-  int64_t printed = (int64_t)covered;
+  const bool sam = p->out_format == 1;
+  int bias = 0;
+  const bool fast_ok = fast_params_ok(Q, R, p->match, p->mismatch, p->gap_open, p->gap_ext, &bias);
+  // Gapless pass over every record (ungapped.cu): `all` is the output's view
+  ReadPackArgs rp;
+  memset(&rp, 0, sizeof(rp));
+  rp.reads = d_reads;
+  rp.rd = d_rd;
+  rp.n_reads = 2 * n;
+  rp.Q = Q;
+  rp.words = code_words(Q);
+  const int max_mis = gapless_max_mismatches(p->match, p->mismatch, p->gap_open, p->gap_ext);
+  const bool gapless = fast_ok && max_mis >= 0 && idx->d_odd && covered > 0;
+  FormatArgs all;
+  memset(&all, 0, sizeof(all));
+  all.reads = d_reads;
+  all.rd = d_rd;
+  all.recs = idx->d_recs;
+  all.cat = (const char*)idx->d_cat;
+  all.Q = Q;
+  all.n = covered;
+  DevPair* all_pairs;
+  DevAln* all_aln;
+  CK(sc.get(&all_pairs, nr));
+  CK(sc.get(&all_aln, nr));
+  all.pairs = all_pairs;
+  all.aln = all_aln;
+  // mate pairing: runs of records of one read (by name), for all records
+  PairSelArgs ps;
+  memset(&ps, 0, sizeof(ps));
+  int32_t* keep;
+  int8_t* sep;
+  uint32_t *run_flag, *run_of, *n_runs_d;
+  int64_t* first;
+  CK(sc.get(&keep, nr));
+  CK(sc.get(&sep, nr));
+  CK(sc.get(&run_flag, nr));
+  CK(sc.get(&run_of, nr));
+  CK(sc.get(&n_runs_d, 1));
+  CK(sc.get(&first, nr));
+  void* tmp3;
+  CK(sc.get((uint8_t**)&tmp3, scan_temp_bytes((int64_t)nrec)));
+  ps.n = covered;
+  ps.pairs = all_pairs;
+  ps.aln = all_aln;
+  ps.id = pa.m_id;
+  ps.batch_start = d_bs;
+  ps.reads = d_reads;
+  ps.rd = d_rd;
+  ps.min_frag = min_frag;
+  ps.max_frag = max_frag;
+  ps.keep = keep;
+  ps.sep = sep;
   if (!sam && covered > 0) {
     // reference-name classes (the pairing compares names, not indices)
     std::vector<int32_t> h_class(idx->recs.size());
@@ -3227,47 +3154,235 @@ static int align_paired_impl(swift_ctx* ctx, const swift_index* idx, const char*
           break;
         }
     }
-    uint8_t* d_bs;
     int32_t* d_class;
-    uint32_t *run_flag, *run_of, *n_runs_d;
-    int64_t* first;
-    void* tmp3;
-    CK(sc.get(&d_bs, nr));
     CK(sc.get(&d_class, std::max<size_t>(h_class.size(), 1)));
-    CK(sc.get(&run_flag, nr));
-    CK(sc.get(&run_of, nr));
-    CK(sc.get(&n_runs_d, 1));
-    CK(sc.get(&first, nr));
-    CK(sc.get((uint8_t**)&tmp3, scan_temp_bytes((int64_t)nrec)));
-    CK(cudaMemcpyAsync(d_bs, h_bs.data(), covered, cudaMemcpyHostToDevice, st));
     CK(cudaMemcpyAsync(d_class, h_class.data(), h_class.size() * 4, cudaMemcpyHostToDevice, st));
-    PairSelArgs ps;
-    memset(&ps, 0, sizeof(ps));
-    ps.n = (int64_t)covered;
-    ps.pairs = pairs;
-    ps.aln = aln;
-    ps.id = pa.m_id;
-    ps.batch_start = d_bs;
-    ps.reads = d_reads;
-    ps.rd = d_rd;
     ps.ref_class = d_class;
-    ps.min_frag = min_frag;
-    ps.max_frag = max_frag;
-    ps.keep = keep;
-    ps.sep = sep;
+  }
+  auto find_runs = [&]() -> int {
     launch_pe_runs(st, ps, run_flag);
     CKLAUNCH();
-    launches += 1 + exclusive_scan_u32(st, run_flag, run_of, (int64_t)covered, tmp3, n_runs_d);
-    uint32_t n_runs = 0;
-    CK(cudaMemcpyAsync(&n_runs, n_runs_d, 4, cudaMemcpyDeviceToHost, st));
+    launches += 2 + exclusive_scan_u32(st, run_flag, run_of, covered, tmp3, n_runs_d);
     launch_pe_run_first(st, ps, run_flag, run_of, first);
     CKLAUNCH();
-    CK(cudaStreamSynchronize(st));
-    launch_pe_pair_runs(st, ps, first, (int64_t)n_runs);
+    return SWIFT_OK;
+  };
+  // the records left to the Smith-Waterman passes
+  int64_t left_n = covered;
+  PairedArgs pl = pa;
+  int32_t* l_of = nullptr;
+  if (gapless) {
+    CK(sc.get(&rp.read_cls, (size_t)std::max<int64_t>(2 * n, 1)));
+    CK(sc.get(&rp.codes, (size_t)std::max<int64_t>(2 * n, 1) * 2 * rp.words));
+    launch_pack_reads(st, rp);
+    CKLAUNCH();
+    GaplessArgs ga;
+    memset(&ga, 0, sizeof(ga));
+    ga.codes = rp.codes;
+    ga.read_cls = rp.read_cls;
+    ga.words = rp.words;
+    ga.ref = idx->d_packed;
+    ga.ref_words = (int64_t)((idx->cat_len + 15) / 16) + 2;
+    ga.odd = idx->d_odd;
+    ga.recs = idx->d_recs;
+    ga.m_read = pa.m_read;
+    ga.m_strand = pa.m_rev;
+    ga.m_ri = pa.m_ri;
+    ga.m_rp = pa.m_off;
+    ga.n = covered;
+    ga.Q = Q;
+    ga.R = R;
+    ga.back = Q;
+    ga.match = p->match;
+    ga.mismatch = p->mismatch;
+    ga.gap_open = p->gap_open;
+    ga.max_mis = max_mis;
+    ga.pairs = all_pairs;
+    ga.aln = all_aln;
+    uint32_t *open, *at, *n_left;
+    CK(sc.get(&ga.state, nr));
+    CK(sc.get(&open, nr));
+    CK(sc.get(&at, nr));
+    CK(sc.get(&n_left, 1));
+    launch_gapless(st, ga);
+    CKLAUNCH();
+    launches += 3;
+    if (sam) {
+      launch_open(st, ga.state, covered, open);
+    } else {
+      rc = find_runs();
+      if (rc != SWIFT_OK) return rc;
+      PairSelArgs before = ps;
+      before.state = ga.state;
+      before.bound = p->match * Q + p->gap_open;
+      before.open = open;
+      launch_pe_pair_runs(st, before, first, n_runs_d);
+      ps.open = open;
+    }
+    CKLAUNCH();
+    launches += 1 + exclusive_scan_u32(st, open, at, covered, tmp3, n_left);
+    uint32_t h_left = 0;
+    CK(rb.get(&h_left, n_left, 4));
+    CK(rb.sync());
+    left_n = h_left;
+    all.src = at;
+    const size_t nl = (size_t)std::max<int64_t>(left_n, 1);
+    LeftArgs left;
+    memset(&left, 0, sizeof(left));
+    left.n = left_n > 0 ? covered : 0;
+    left.open = open;
+    left.at = at;
+    left.m_read = pa.m_read;
+    left.m_strand = pa.m_rev;
+    left.m_ri = pa.m_ri;
+    left.m_rp = pa.m_off;
+    CK(sc.get(&left.l_read, nl));
+    CK(sc.get(&left.l_strand, nl));
+    CK(sc.get(&left.l_ri, nl));
+    CK(sc.get(&left.l_rp, nl));
+    CK(sc.get(&left.l_of, nl));
+    launch_left(st, left);
+    CKLAUNCH();
+    launches += left_n > 0 ? 1 : 0;
+    pl.m_read = left.l_read;
+    pl.m_rev = left.l_strand;
+    pl.m_ri = left.l_ri;
+    pl.m_off = left.l_rp;
+    l_of = left.l_of;
+  }
+  // Phase 2 pairs: query Q, window 3Q; the packed passes trace pairs of
+  // ACGT bytes with full windows, the generic kernel the others
+  const size_t nl = (size_t)std::max<int64_t>(left_n, 1);
+  const int64_t qs = (Q + 16) & ~15, ws = (R + 16) & ~15;
+  const int64_t cs = ((int64_t)Q + R + 2 + 15) & ~(int64_t)15;  // the walk stores words
+  char *qbuf, *wbuf, *qcons, *rcons;
+  DevPair* pairs = all_pairs;
+  DevAln* aln = all_aln;
+  CK(sc.get(&qbuf, nl * qs));
+  CK(sc.get(&wbuf, nl * ws));
+  CK(sc.get(&qcons, nl * cs));
+  CK(sc.get(&rcons, nl * cs));
+  if (gapless) {
+    CK(sc.get(&pairs, nl));
+    CK(sc.get(&aln, nl));
+  }
+  CK(cudaMemsetAsync(wbuf, 0, nl * ws, st));
+  pl.n_rec = left_n;
+  pl.Q = Q;
+  pl.ref_file = idx->d_file;
+  pl.cat = (const char*)idx->d_cat;
+  pl.odd = idx->d_odd;
+  pl.ref_file_len = idx->file_len;
+  pl.recs = idx->d_recs;
+  pl.reads = d_reads;
+  pl.rd = d_rd;
+  pl.pairs = pairs;
+  pl.qbuf = qbuf;
+  pl.wbuf = wbuf;
+  pl.q_stride = qs;
+  pl.w_stride = ws;
+  launch_pe_pairs(st, pl);
+  CKLAUNCH();
+  launches += left_n > 0 ? 1 : 0;
+  CK(cudaEventRecord(ctx->ev[2], st));
+  int32_t *fast_list, *gen_list, *lcnt;
+  CK(sc.get(&fast_list, nl));
+  CK(sc.get(&gen_list, nl));
+  CK(sc.get(&lcnt, 2));
+  CK(cudaMemsetAsync(lcnt, 0, 2 * sizeof(int32_t), st));
+  if (left_n > 0) {
+    partition_pairs_kernel<<<(unsigned)((left_n + 255) / 256), 256, 0, st>>>(
+        pairs, left_n, fast_ok ? 0 : 1, fast_list, lcnt, gen_list, lcnt + 1);
+    CKLAUNCH();
+    ++launches;
+    SwArgs sa;
+    memset(&sa, 0, sizeof(sa));
+    sa.q = qbuf;
+    sa.w = wbuf;
+    sa.q_stride = qs;
+    sa.w_stride = ws;
+    sa.Q = Q;
+    sa.R = R;
+    sa.match = p->match;
+    sa.mismatch = p->mismatch;
+    sa.gap_open = p->gap_open;
+    sa.gap_ext = p->gap_ext;
+    sa.n = left_n;
+    sa.aln = aln;
+    sa.qcons = qcons;
+    sa.rcons = rcons;
+    sa.cons_stride = cs;
+    sa.list = gen_list;
+    sa.count = lcnt + 1;
+    rc = launch_sw(st, sa, &ctx->err);
+    if (rc != SWIFT_OK) return rc;
+    CKLAUNCH();
+    ++launches;
+    if (fast_ok) {
+      const int64_t chunk = 262144;
+      // (grids are sized by the records left; the kernels read the list's length)
+      int2* best2;
+      uint32_t* dirs;
+      CK(sc.get(&best2, nl));
+      CK(sc.get(&dirs, (size_t)trace_scratch_words(Q, R, std::min<int64_t>(left_n, chunk))));
+      FastArgs fa2;
+      memset(&fa2, 0, sizeof(fa2));
+      fa2.q = qbuf;
+      fa2.w = wbuf;
+      fa2.q_stride = qs;
+      fa2.w_stride = ws;
+      fa2.Q = Q;
+      fa2.R = R;
+      fa2.match = p->match;
+      fa2.mismatch = p->mismatch;
+      fa2.gap_open = p->gap_open;
+      fa2.gap_ext = p->gap_ext;
+      fa2.bias = bias;
+      fa2.aln = aln;
+      fa2.qcons = qcons;
+      fa2.rcons = rcons;
+      fa2.cons_stride = cs;
+      fa2.best = best2;
+      fa2.list = fast_list;
+      fa2.count = lcnt;
+      fa2.dirs = dirs;
+      for (int64_t off = 0; off < left_n; off += chunk) {
+        fa2.list_offset = off;
+        const int kk = launch_sw_trace(st, fa2, std::min<int64_t>(chunk, left_n - off));
+        if (kk == 0) return fail(ctx, SWIFT_E_DEVICE, "trace pass could not launch");
+        launches += kk;
+        CKLAUNCH();
+      }
+    }
+    if (gapless) {
+      launch_put_back(st, l_of, aln, nullptr, left_n, all_aln, nullptr);
+      CKLAUNCH();
+      ++launches;
+    }
+  }
+  CK(cudaEventRecord(ctx->ev[3], st));
+  FormatArgs fa = all;
+  fa.qcons = qcons;
+  fa.rcons = rcons;
+  fa.cons_stride = cs;
+  uint64_t *bytes, *offs, *tot2;
+  void* tmp2;
+  CK(sc.get(&bytes, nr));
+  CK(sc.get(&offs, nr));
+  CK(sc.get(&tot2, 1));
+  CK(sc.get((uint8_t**)&tmp2, scan_temp_bytes((int64_t)nrec)));
+  int64_t printed = covered;
+  if (!sam && covered > 0) {
+    // selection (chooseBestAlignment_paired3 per batch) of the steps open
+    if (!gapless) {
+      rc = find_runs();
+      if (rc != SWIFT_OK) return rc;
+    }
+    launch_pe_pair_runs(st, ps, first, n_runs_d);
     CKLAUNCH();
     launch_pe_sep(st, ps);
     CKLAUNCH();
-    launches += 3;
+    launches += 2;
     fa.keep = keep;
     fa.pe_sep = sep;
   }
@@ -3281,7 +3396,6 @@ static int align_paired_impl(swift_ctx* ctx, const swift_index* idx, const char*
   CKLAUNCH();
   launches += (covered > 0 ? 1 : 0) + exclusive_scan_u64(st, bytes, offs, (int64_t)covered, tmp2, tot2);
   uint64_t total = 0;
-  Readback rb(ctx);
   CK(rb.get(&total, tot2, 8));
   TextChunks chunks;
   rc = chunks.plan(ctx, rb, offs, (int64_t)covered, host_out != nullptr);

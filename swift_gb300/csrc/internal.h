@@ -354,8 +354,6 @@ struct GaplessArgs {
   const int32_t* m_strand;
   const int32_t* m_ri;
   const int32_t* m_rp;
-  const int32_t* m_mate;      // optional: mate 2's reads start at mate2
-  int32_t mate2;
   int64_t n;
   int Q;
   const int32_t* read_q;      // optional: query length per read
@@ -397,7 +395,7 @@ struct PairedArgs {
   const int3 *best1, *best2;
   const uint64_t* roff;       // per pair: first record
   int64_t n_rec;
-  int32_t *m_id, *m_mate, *m_rev, *m_read, *m_ri, *m_shift, *m_off;
+  int32_t *m_id, *m_rev, *m_read, *m_ri, *m_shift, *m_off;  // m_read: mate 2's after mate 1's
   int Q;
   const char* ref_file;
   uint64_t ref_file_len;
@@ -429,6 +427,10 @@ struct PairSelArgs {
   const DevRead* rd;
   const int32_t* ref_class;   // per reference: its name's class (equal names, equal class)
   uint32_t min_frag, max_frag;
+  const uint8_t* state;       // before the Smith-Waterman passes: the gapless pass's
+  int bound;                  // its bound of an unsettled score
+  uint32_t* open;             // per record: 1 left to the Smith-Waterman passes
+                              // (written before them, optional after)
   int32_t* keep;              // out: printed
   int8_t* sep;                // out: 1 opens with the line of '*'
 };
@@ -436,7 +438,7 @@ void launch_pe_runs(cudaStream_t st, const PairSelArgs& a, uint32_t* flag);
 void launch_pe_run_first(cudaStream_t st, const PairSelArgs& a, const uint32_t* flag,
                          const uint32_t* run_of, int64_t* first);
 void launch_pe_pair_runs(cudaStream_t st, const PairSelArgs& a, const int64_t* first,
-                         int64_t n_runs);
+                         const uint32_t* n_runs);
 void launch_pe_sep(cudaStream_t st, const PairSelArgs& a);
 
 // sw.cu

@@ -36,9 +36,8 @@ __global__ void pe_fill_kernel(PairedArgs a) {
       for (int h = 0; h < nb[sid]; ++h) {
         const int3 b = best[sid * a.max_hits + h];
         a.m_id[o] = (int32_t)(i + 1);
-        a.m_mate[o] = mate + 1;
         a.m_rev[o] = s;
-        a.m_read[o] = (int32_t)i;
+        a.m_read[o] = (int32_t)(mate * a.n_pairs + i);
         a.m_ri[o] = b.x;
         a.m_shift[o] = b.y;
         a.m_off[o] = b.z;
@@ -61,7 +60,7 @@ __global__ void __launch_bounds__(kPeWarps * 32) pe_pairs_kernel(PairedArgs a) {
   const int64_t j = (int64_t)blockIdx.x * kPeWarps + (threadIdx.x >> 5);
   if (j >= a.n_rec) return;
   const int Q = a.Q, R = 3 * a.Q;
-  const int mate = a.m_mate[j], rev = a.m_rev[j], read = a.m_read[j], ri = a.m_ri[j];
+  const int rev = a.m_rev[j], cr = a.m_read[j], ri = a.m_ri[j];
   int dist = a.m_off[j] - Q;
   if (dist < 0) dist = 0;
   const DevRecord& rec = a.recs[ri];
@@ -126,7 +125,6 @@ __global__ void __launch_bounds__(kPeWarps * 32) pe_pairs_kernel(PairedArgs a) {
   }
   if (got > R) got = R;
   // query: the mate's read, first Q bases
-  const int64_t cr = mate == 1 ? (int64_t)read : a.n_pairs + read;
   const DevRead rr = a.rd[cr];
   const char* s = a.reads + rr.seq_off;
   char* q = a.qbuf + j * a.q_stride;
@@ -147,7 +145,7 @@ __global__ void __launch_bounds__(kPeWarps * 32) pe_pairs_kernel(PairedArgs a) {
   odd = __any_sync(0xffffffffu, odd);
   if (lane == 0) {
     DevPair p;
-    p.read = (int32_t)cr;
+    p.read = cr;
     p.strand = rev;
     p.ref_idx = ri;
     p.ref_dist = dist;
@@ -249,10 +247,21 @@ __device__ __forceinline__ bool frag_ok(const PairSelArgs& a, int64_t i, int64_t
   return (uint32_t)d >= a.min_frag && (uint32_t)d <= a.max_frag;
 }
 
-// per run: the pairing step it starts, if it starts one
-__global__ void pe_pair_runs_kernel(PairSelArgs a, const int64_t* first, int64_t n_runs) {
-  const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+// Per run: the pairing step it starts, if it starts one.
+//
+// Before the Smith-Waterman passes (a.state given): the steps the gapless
+// pass settles.  A run without its mate prints nothing, whatever its scores.
+// Otherwise, with every record of the step looked at, let S be the largest
+// sum of a settled pair that may be printed.  A pair with an unsettled record
+// sums to at most a.bound (an unsettled score's bound) plus the larger of
+// a.bound and the other run's largest settled score; when S lies above that,
+// the first settled pair of sum S is the step's pick and no other score is
+// needed.  The records of the other steps are left open (a.open).
+// After them (a.state null): the open steps.
+__global__ void pe_pair_runs_kernel(PairSelArgs a, const int64_t* first, const uint32_t* n_runs_d) {
+  const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, n_runs = *n_runs_d;
   if (r >= n_runs) return;
+  const bool before = a.state != nullptr;
   // m(h): run h's next run lies in its batch and carries its mate core
   auto run_end = [&](int64_t h) { return h + 1 < n_runs ? first[h + 1] : a.n; };
   auto mates = [&](int64_t h) {
@@ -266,26 +275,47 @@ __global__ void pe_pair_runs_kernel(PairSelArgs a, const int64_t* first, int64_t
   // runs h + 1 .. r - 1 all pair with their next run: steps alternate
   if (((r - h - 1) & 1) != 0) return;  // run r is the mate run of r - 1
   const int64_t s1 = first[r], e1 = run_end(r);
+  if (!before && a.open && !a.open[s1]) return;
   if (!mates(r)) {
-    for (int64_t i = s1; i < e1; ++i) a.keep[i] = 0;
+    for (int64_t i = s1; i < e1; ++i) {
+      a.keep[i] = 0;
+      if (before) a.open[i] = 0;
+    }
     return;
   }
   const int64_t s2 = e1, e2 = run_end(r + 1);
+  auto known = [&](int64_t i) { return !before || a.state[i] == kGaplessDone; };
   int best = 0;
-  for (int64_t i = s1; i < e1; ++i)
+  for (int64_t i = s1; i < e1; ++i) {
+    if (!known(i)) continue;
     for (int64_t j = s2; j < e2; ++j) {
-      if (!opposite(a, i, j)) continue;
+      if (!known(j) || !opposite(a, i, j)) continue;
       const int sum = a.aln[i].score + a.aln[j].score;
       if (best < sum && frag_ok(a, i, j)) best = sum;
     }
+  }
+  if (before) {
+    bool all = true;
+    int most = a.bound;
+    for (int64_t i = s1; i < e2; ++i) {
+      all = all && a.state[i] != kGaplessOther;
+      if (a.state[i] == kGaplessDone) most = max(most, a.aln[i].score);
+    }
+    const uint32_t open = all && best > a.bound + most ? 0u : 1u;
+    for (int64_t i = s1; i < e2; ++i) a.open[i] = open;
+    if (open) return;
+  }
   int64_t f1 = -1, f2 = -1;
-  for (int64_t i = s1; i < e1 && f1 < 0; ++i)
+  for (int64_t i = s1; i < e1 && f1 < 0; ++i) {
+    if (!known(i)) continue;
     for (int64_t j = s2; j < e2; ++j)
-      if (opposite(a, i, j) && a.aln[i].score + a.aln[j].score == best && frag_ok(a, i, j)) {
+      if (known(j) && opposite(a, i, j) && a.aln[i].score + a.aln[j].score == best &&
+          frag_ok(a, i, j)) {
         f1 = i;
         f2 = j;
         break;
       }
+  }
   for (int64_t i = s1; i < e1; ++i) a.keep[i] = i == f1 ? 1 : 0;
   for (int64_t j = s2; j < e2; ++j) a.keep[j] = j == f2 ? 1 : 0;
 }
@@ -368,9 +398,9 @@ void launch_pe_run_first(cudaStream_t st, const PairSelArgs& a, const uint32_t* 
 }
 
 void launch_pe_pair_runs(cudaStream_t st, const PairSelArgs& a, const int64_t* first,
-                         int64_t n_runs) {
-  if (n_runs <= 0) return;
-  pe_pair_runs_kernel<<<(unsigned)((n_runs + 127) / 128), 128, 0, st>>>(a, first, n_runs);
+                         const uint32_t* n_runs) {
+  if (a.n <= 0) return;
+  pe_pair_runs_kernel<<<(unsigned)((a.n + 127) / 128), 128, 0, st>>>(a, first, n_runs);
 }
 
 void launch_pe_sep(cudaStream_t st, const PairSelArgs& a) {

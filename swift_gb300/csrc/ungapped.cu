@@ -123,8 +123,7 @@ constexpr int kGaplessThreads = 128;
 __global__ void __launch_bounds__(kGaplessThreads) gapless_kernel(GaplessArgs a) {
   const int64_t j = (int64_t)blockIdx.x * kGaplessThreads + threadIdx.x;
   if (j >= a.n) return;
-  const int32_t strand = a.m_strand[j], ri = a.m_ri[j];
-  const int32_t read = a.m_read[j] + (a.m_mate && a.m_mate[j] == 2 ? a.mate2 : 0);
+  const int32_t read = a.m_read[j], strand = a.m_strand[j], ri = a.m_ri[j];
   const int32_t dist = max(0, a.m_rp[j] - a.back);
   const DevRecord& rec = a.recs[ri];
   const int Q = a.read_q ? a.read_q[read] : a.Q, R = a.R;

@@ -176,3 +176,34 @@ def test_reads_settled_without_smith_waterman(ctx, sg):
     got, st = ctx.align(ctx.index(fasta([s])), reads, stats=True)
     assert st["printed"] == 1024 == st["traced_pairs"]
     assert st["sw_cells_computed"] == 0 and got.count(b"Score: 200.0") == 1024
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("L,frag", [(36, (50, 400)), (64, (99, 600)), (100, (180, 320))])
+def test_paired_steps(ctx, sg, oracle, L, frag):
+    # mate pairs with 0-6 substitutions among repeats: steps settled whole,
+    # steps with one unsettled mate, sums that tie, fragments at the limits
+    rng = random.Random(900 + L)
+    rand = lambda k: bytes(rng.choice(b"ACGT") for _ in range(k))
+    unit = rand(400)
+    s = rand(900) + unit + rand(300) + unit + mutated(rng, unit, 3, False) + rand(900)
+    r1, r2 = [], []
+    for i in range(300):
+        f = rng.choice([rng.randint(L, 500), frag[0], frag[1], frag[0] - 1, frag[1] + 1])
+        f = max(f, L)
+        at = rng.randrange(len(s) - f)
+        a = mutated(rng, s[at:at + L], i % 4, i % 13 == 4)
+        b = mutated(rng, s[at + f - L:at + f], i % 7, False)
+        if i % 10 == 9:
+            b = rand(L)
+        m1, m2 = (a + rand(L))[:L], revcomp((b + rand(L))[:L])
+        if i % 5 == 2:
+            m1, m2 = m2, m1
+        r1.append(b">p%d/1\n%s\n" % (i, m1))
+        r2.append(b">p%d/2\n%s\n" % (i, m2))
+    r1, r2, ref = b"".join(r1), b"".join(r2), fasta([s])
+    ix = ctx.index(ref)
+    for fmt in (0, 1):
+        got = ctx.align_paired(ix, r1, r2, sg.default_params(out_format=fmt), *frag)
+        o = oracle.default_params(device_mem=ctx.info()["total_mem"], out_format=fmt)
+        assert got == oracle.align_paired(ref, r1, r2, o, *frag)

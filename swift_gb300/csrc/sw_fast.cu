@@ -174,7 +174,8 @@ int launch_sw_score(cudaStream_t st, const FastArgs& a, int64_t max_pairs) {
 
 int launch_sw_trace(cudaStream_t st, const FastArgs& a, int64_t max_pairs, cudaEvent_t before,
                     cudaEvent_t after) {
-  if (a.cons_stride % 4 != 0) return 0;  // the walk stores 32-bit words
+  // the walk stores 32-bit words, and reads words of the query and window rows
+  if (a.cons_stride % 4 != 0 || (a.q_stride | a.w_stride) % 4 != 0) return 0;
   FastArgs b = a;
   b.chunk = max_pairs;
   b.one = 1;

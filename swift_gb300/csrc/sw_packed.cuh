@@ -470,18 +470,42 @@ __global__ void __launch_bounds__(kPkWarps * 32, (TRACE || RPL > 13) ? 16 / kPkW
 }
 
 // Traceback walk (src/smithWaterman.cu:911-1026), one thread per printed
-// pair: dependent loads of the 4-bit directions the trace pass streamed out;
-// many walks in flight hide each other's latency.
+// pair over the 2-bit directions the trace pass streamed out.
+//
+// Each move depends on the one before, so a walk is bound by the latency of
+// its loads.  A warp's walks refill together: a round copies into shared
+// memory everything the next kWalkMoves moves of a walk can touch (the last
+// kWalkMoves + 1 steps of its lane's direction stream and of the streams of
+// the lanes above that it can reach, the query and window bytes before its
+// cell), all of it loads that do not wait for one another, and the moves then
+// run from shared memory.  (With each walk refilling a register cache when it
+// left it, some walk of a warp waited for memory on almost every move: 10,000
+// reads' walks took 125 us, with rounds 51 us; more moves a round load more
+// than the walks use.)
 constexpr int kWalkThreads = 128;  // small blocks: walks of uneven length leave SMs sooner
+constexpr int kWalkMoves = 8;
+
+template <int G, int RPL>
+struct WalkRound {
+  static constexpr int kNW = DirLayout<RPL>::kWords;
+  static constexpr int kStreams = (kWalkMoves + RPL - 1) / RPL + 1;
+  // 16-byte blocks of a stream: its words and up to 3 before them
+  static constexpr int kBlocks = ((kWalkMoves + 1) * kNW + 3 + 3) / 4;
+  static constexpr int kSeq = (kWalkMoves + 3 + 3) / 4;  // words of query or window bytes
+  static constexpr int kWordsAll = kStreams * kBlocks * 4 + 2 * kSeq;
+};
 
 template <int G, int RPL>
 __global__ void __launch_bounds__(kWalkThreads) sw_walk_kernel(FastArgs a) {
+  using Round = WalkRound<G, RPL>;
   constexpr int kGroups = 32 / G;
   constexpr int kPairs = 2 * kGroups;
-  constexpr int kNW = DirLayout<RPL>::kWords;
+  constexpr int kNW = Round::kNW;
+  // [word][thread]: a thread's words never share a bank with another's
+  __shared__ uint32_t sh[Round::kWordsAll * kWalkThreads];
   const int64_t nlist = *a.count - a.list_offset;
   const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= nlist || idx >= a.chunk) return;
+  if (idx >= nlist || idx >= a.chunk) return;  // (no block-wide synchronisation below)
   const int32_t p = a.list[a.list_offset + idx];
   const int64_t warp = idx / kPairs;
   const int g = (int)((idx % kPairs) >> 1);
@@ -493,59 +517,8 @@ __global__ void __launch_bounds__(kWalkThreads) sw_walk_kernel(FastArgs a) {
   const char* wg = a.w + (int64_t)p * a.w_stride;
   const int W = (a.r_len ? a.r_len[p] : R) + 1;  // the pair's own window for cell indices
   const int shift_half = 16 * hp;
-  // The walk moves to lower addresses one step (kNW words) per diagonal
-  // move inside a lane's rows: the direction words are kept as three
-  // 16-byte blocks in registers, the one holding the cell's word and the two
-  // before it, so one round of loads serves several steps instead of one
-  // dependent load per step.  (The group's region starts 16-byte aligned and
-  // holds at least 16 blocks; blocks below its start are never read.)
-  const uint4* dirs4 = reinterpret_cast<const uint4*>(dirs);
-  int64_t blk = -16;  // first cached block
-  uint4 c0 = make_uint4(0, 0, 0, 0), c1 = c0, c2 = c0;
-  auto pick = [](const uint4& v, int w) -> uint32_t {
-    return w == 0 ? v.x : w == 1 ? v.y : w == 2 ? v.z : v.w;
-  };
-  // the 2-bit code (2 UP, 1 LEFT, 0 DIAG or NONE) of the cell in row
-  // ln * RPL + k + 1 (lane ln, its row k) and column jj: word
-  // (ln * S8 + jj + ln - 1) * kNW + k / 8 of the lane streams
-  auto code_at = [&](int ln, int k, int jj) -> uint32_t {
-    const int64_t at = ((int64_t)ln * S8 + (jj + ln - 1)) * kNW + (k >> 3);
-    const int64_t b = at >> 2;
-    if (b < blk || b > blk + 2) {
-      blk = b >= 2 ? b - 2 : 0;
-      c0 = __ldg(dirs4 + blk);
-      c1 = __ldg(dirs4 + blk + 1);
-      c2 = __ldg(dirs4 + blk + 2);
-    }
-    const int o = (int)(b - blk), w = (int)(at & 3);
-    const uint32_t word = o == 0 ? pick(c0, w) : o == 1 ? pick(c1, w) : pick(c2, w);
-    const int rows_w = min(8, RPL - (k & ~7));  // rows of the word, the last lowest
-    return (word >> (shift_half + 2 * (rows_w - 1 - (k & 7)))) & 3u;
-  };
-  // query and window bytes in 16-byte blocks too (rows start 16-byte
-  // aligned, strides are multiples of 16)
-  const bool blocks16 = ((a.q_stride | a.w_stride) & 15) == 0;
-  int qb = -1, wb = -1;
-  uint4 q16 = make_uint4(0, 0, 0, 0), w16 = q16;
-  auto byte_of = [&](const uint4& v, int o) -> char {
-    return (char)((pick(v, o >> 2) >> (8 * (o & 3))) & 0xFFu);
-  };
-  auto qbyte = [&](int i) -> char {
-    if (!blocks16) return qg[i];
-    if ((i >> 4) != qb) {
-      qb = i >> 4;
-      q16 = __ldg(reinterpret_cast<const uint4*>(qg) + qb);
-    }
-    return byte_of(q16, i & 15);
-  };
-  auto wbyte = [&](int i) -> char {
-    if (!blocks16) return wg[i];
-    if ((i >> 4) != wb) {
-      wb = i >> 4;
-      w16 = __ldg(reinterpret_cast<const uint4*>(wg) + wb);
-    }
-    return byte_of(w16, i & 15);
-  };
+  uint32_t* mine = sh + threadIdx.x;
+  const char* bytes = reinterpret_cast<const char*>(mine + Round::kStreams * Round::kBlocks * 4 * kWalkThreads);
   // consensus bytes are gathered four at a time and stored as words
   // (consensus strings are optional: coordinates only when qcons is null)
   const bool cons = a.qcons != nullptr;
@@ -566,49 +539,107 @@ __global__ void __launch_bounds__(kWalkThreads) sw_walk_kernel(FastArgs a) {
   int h = b.x;                     // its score
   // its lane and row in the lane (kept as the walk moves up)
   int ln = cr > 0 ? (cr - 1) / RPL : 0, k = cr > 0 ? (cr - 1) % RPL : 0;
-  int d = (cr == 0 || cc == 0) ? kNone : dir_of(code_at(ln, k, cc), h);
-  // One move per step: its consensus bytes (a gap where the row or column
-  // stays), then, unless it reached row or column 0, the predecessor's
-  // score (the substitution score for a DIAG move; for a gap, gap_ext when
-  // the predecessor itself moved the same way, else gap_open) and
-  // direction.  The walk ends at a NONE cell or at the border.
+  int d = (cr == 0 || cc == 0) ? kNone : kDiag;  // the first round reads the cell's own
+  bool fresh = true;
   int tick = -1, nref = -1, start = 0;
   while (d != kNone) {
-    const bool up = d != kLeft, left = d != kUp;  // row / column move
-    const char qc = qbyte(cr - 1), rc = wbyte(cc - 1);
-    ++tick;
-    nref += left ? 1 : 0;
-    {
-      const int sh = 8 * (tick & 3);
-      racc |= (uint32_t)(uint8_t)(left ? rc : '-') << sh;
-      qacc |= (uint32_t)(uint8_t)(up ? qc : '-') << sh;
-      if ((tick & 3) == 3) {
-        if (cons) {
-          rcw[tick >> 2] = racc;
-          qcw[tick >> 2] = qacc;
+    // the round's words: stream t holds lane ln - t from word base(t) on
+    const int ln0 = ln, step_lo = cc - kWalkMoves + ln - 1;  // lane ln's earliest step
+    auto base = [&](int t) -> int {
+      const int lane0 = (ln0 - t) * S8, lo = step_lo - t;
+      return ((lane0 + max(lo, 0)) * kNW) & ~3;
+    };
+#pragma unroll
+    for (int t = 0; t < Round::kStreams; ++t) {
+      if (ln0 - t >= 0) {
+        const uint4* src = reinterpret_cast<const uint4*>(dirs + base(t));
+        uint4 v[Round::kBlocks];
+        // (blocks past a stream's last step lie in the next lane's stream or
+        // the scratch's spare groups)
+#pragma unroll
+        for (int q = 0; q < Round::kBlocks; ++q) v[q] = __ldg(src + q);
+#pragma unroll
+        for (int q = 0; q < Round::kBlocks; ++q) {
+          uint32_t* to = mine + (t * Round::kBlocks + q) * 4 * kWalkThreads;
+          to[0] = v[q].x;
+          to[kWalkThreads] = v[q].y;
+          to[2 * kWalkThreads] = v[q].z;
+          to[3 * kWalkThreads] = v[q].w;
         }
-        racc = qacc = 0;
       }
     }
-    start = cc;
-    const int nr = cr - (up ? 1 : 0), nc = cc - (left ? 1 : 0);
-    if (nr == 0 || nc == 0) break;
-    if (up && --k < 0) {
-      k = RPL - 1;
-      --ln;
+    // query rows and window columns before the cell, from 4-byte words (rows
+    // of the buffers start 16-byte aligned)
+    const int q0 = max(cr - kWalkMoves, 0) & ~3, w0 = max(cc - kWalkMoves, 0) & ~3;
+    {
+      const uint32_t* qs = reinterpret_cast<const uint32_t*>(qg + q0);
+      const uint32_t* ws = reinterpret_cast<const uint32_t*>(wg + w0);
+      uint32_t* to = mine + Round::kStreams * Round::kBlocks * 4 * kWalkThreads;
+#pragma unroll
+      for (int q = 0; q < Round::kSeq; ++q) {
+        // (words past the cell's are not needed and may lie past the row)
+        to[q * kWalkThreads] = q0 + 4 * q < cr ? __ldg(qs + q) : 0u;
+        to[(Round::kSeq + q) * kWalkThreads] = w0 + 4 * q < cc ? __ldg(ws + q) : 0u;
+      }
     }
-    const uint32_t pc = code_at(ln, k, nc);
-    int nh;
-    if (d == kDiag) {
-      const char uq = upc(qc), ur = upc(rc);
-      nh = h - ((uq == ur || uq == 'N' || ur == 'N') ? m : x);
-    } else {
-      nh = h - ((d == kUp ? pc == 2u : pc == 1u) ? e : o);
+    auto byte_at = [&](int w, int i) -> char {
+      return bytes[(w + (i >> 2)) * 4 * kWalkThreads + (i & 3)];
+    };
+    // the 2-bit code (2 UP, 1 LEFT, 0 DIAG or NONE) of the cell in lane l's
+    // row kk and column jj
+    auto code_at = [&](int l, int kk, int jj) -> uint32_t {
+      const int t = ln0 - l;
+      const int at = (l * S8 + (jj + l - 1)) * kNW + (kk >> 3) - base(t);
+      const uint32_t word = mine[(t * Round::kBlocks * 4 + at) * kWalkThreads];
+      const int rows_w = min(8, RPL - (kk & ~7));  // rows of the word, the last lowest
+      return (word >> (shift_half + 2 * (rows_w - 1 - (kk & 7)))) & 3u;
+    };
+    if (fresh) {
+      d = dir_of(code_at(ln, k, cc), h);
+      fresh = false;
     }
-    cr = nr;
-    cc = nc;
-    h = nh;
-    d = dir_of(pc, nh);
+    // One move per step: its consensus bytes (a gap where the row or column
+    // stays), then, unless it reached row or column 0, the predecessor's
+    // score (the substitution score for a DIAG move; for a gap, gap_ext when
+    // the predecessor itself moved the same way, else gap_open) and
+    // direction.  The walk ends at a NONE cell or at the border.
+    for (int mv = 0; mv < kWalkMoves && d != kNone; ++mv) {
+      const bool up = d != kLeft, left = d != kUp;  // row / column move
+      const char qc = byte_at(0, cr - 1 - q0), rc = byte_at(Round::kSeq, cc - 1 - w0);
+      ++tick;
+      nref += left ? 1 : 0;
+      {
+        const int sh8 = 8 * (tick & 3);
+        racc |= (uint32_t)(uint8_t)(left ? rc : '-') << sh8;
+        qacc |= (uint32_t)(uint8_t)(up ? qc : '-') << sh8;
+        if ((tick & 3) == 3) {
+          if (cons) {
+            rcw[tick >> 2] = racc;
+            qcw[tick >> 2] = qacc;
+          }
+          racc = qacc = 0;
+        }
+      }
+      start = cc;
+      cr -= up ? 1 : 0;
+      cc -= left ? 1 : 0;
+      if (cr == 0 || cc == 0) {
+        d = kNone;
+        break;
+      }
+      if (up && --k < 0) {
+        k = RPL - 1;
+        --ln;
+      }
+      const uint32_t pc = code_at(ln, k, cc);
+      if (d == kDiag) {
+        const char uq = upc(qc), ur = upc(rc);
+        h -= (uq == ur || uq == 'N' || ur == 'N') ? m : x;
+      } else {
+        h -= (d == kUp ? pc == 2u : pc == 1u) ? e : o;
+      }
+      d = dir_of(pc, h);
+    }
   }
   if (cons && tick >= 0 && (tick & 3) != 3) {
     rcw[tick >> 2] = racc;

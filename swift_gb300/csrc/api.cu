@@ -2444,6 +2444,26 @@ static int align_resident_impl(swift_ctx* ctx, const swift_index* idx, const swi
   CK(sc.get(&d_cells, 2));
   CK(cudaMemsetAsync(d_cells, 0, 2 * sizeof(unsigned long long), st));
   fa2.cells_done = d_cells;
+  // the generic kernel's pairs: mostly a handful, which take as long as one
+  // does (100 us).  Where the packed pairs are traced at once they run beside
+  // that on the side stream, joined before their results are read (10,000
+  // reads 555 -> 505 us); beside the LCS pass they gained nothing (a million
+  // reads 11.98 -> 12.09 ms).
+  SideJoin generic(ctx);
+  if (n > 0) {
+    const bool beside = fast_ok && (direct || sam);
+    if (beside) {
+      rc = side_fork(ctx);
+      if (rc != SWIFT_OK) return rc;
+      generic.armed = true;
+    }
+    sa.list = gen_list;
+    sa.count = cnt + 1;
+    rc = launch_sw(beside ? ctx->side : st, sa, &ctx->err);
+    if (rc != SWIFT_OK) return rc;
+    CKLAUNCH();
+    ++launches;
+  }
   CK(cudaEventRecord(ctx->ev[7], st));
   if (fast_ok && n > 0 && !sam && !direct) {
     fa2.list = fast_list;
@@ -2457,14 +2477,6 @@ static int align_resident_impl(swift_ctx* ctx, const swift_index* idx, const swi
     CKLAUNCH();
   }
   CK(cudaEventRecord(ctx->ev[8], st));
-  if (n > 0) {
-    sa.list = gen_list;
-    sa.count = cnt + 1;
-    rc = launch_sw(st, sa, &ctx->err);
-    if (rc != SWIFT_OK) return rc;
-    CKLAUNCH();
-    ++launches;
-  }
   CK(cudaEventRecord(ctx->ev[3], st));
   FormatArgs fa = all;
   fa.src = nullptr;
@@ -2490,7 +2502,8 @@ static int align_resident_impl(swift_ctx* ctx, const swift_index* idx, const swi
   auto trace_list = [&](int32_t* list, int32_t* count, int64_t n, bool timed) -> int {
     const int64_t chunk = 262144;
     if (n <= 0) return SWIFT_OK;
-    const int64_t words = trace_scratch_words(Q, kWin, std::min(n, chunk));
+    few_pairs_shape(Q, n, &fa2.shape_g, &fa2.shape_rpl);
+    const int64_t words = trace_scratch_words(Q, kWin, std::min(n, chunk), fa2.shape_g, fa2.shape_rpl);
     uint32_t* dirs;
     CK(sc.get(&dirs, (size_t)words));
     fa2.list = list;
@@ -2623,11 +2636,16 @@ static int align_resident_impl(swift_ctx* ctx, const swift_index* idx, const swi
       fa2.list = ex_list;
       fa2.count = cnt + 3;
       fa2.list_offset = 0;
+      few_pairs_shape(Q, lcs_kept, &fa2.shape_g, &fa2.shape_rpl);
       fa2.cand = cand;
       launches += launch_sw_score(st, fa2, lcs_kept);
       CKLAUNCH();
       fa2.cand = nullptr;
     }
+  }
+  if (generic.armed) {
+    rc = generic.join();
+    if (rc != SWIFT_OK) return rc;
   }
   if (!sam) {
     launch_select(st, fa);
@@ -3324,9 +3342,11 @@ static int align_paired_impl(swift_ctx* ctx, const swift_index* idx, const char*
       int2* best2;
       uint32_t* dirs;
       CK(sc.get(&best2, nl));
-      CK(sc.get(&dirs, (size_t)trace_scratch_words(Q, R, std::min<int64_t>(left_n, chunk))));
       FastArgs fa2;
       memset(&fa2, 0, sizeof(fa2));
+      few_pairs_shape(Q, left_n, &fa2.shape_g, &fa2.shape_rpl);
+      CK(sc.get(&dirs, (size_t)trace_scratch_words(Q, R, std::min<int64_t>(left_n, chunk),
+                                                   fa2.shape_g, fa2.shape_rpl)));
       fa2.q = qbuf;
       fa2.w = wbuf;
       fa2.q_stride = qs;

@@ -591,6 +591,12 @@ __host__ __device__ inline int var_rows(int Q) {
   return Q <= 32 ? 32 : Q <= 128 ? (Q + 7) & ~7 : Q <= 256 ? (Q + 15) & ~15
        : Q <= 320 ? (Q + 31) & ~31 : -1;
 }
+// The shape of a launch of few pairs (0, 0: the default for Q).  Up to
+// kFewPairs pairs (20 a SM) the warps of any shape fit the GPU at once and a
+// launch lasts as long as one warp, whose step costs its rows per lane: more
+// lanes with fewer rows each end sooner, though they do more work in all.
+constexpr int64_t kFewPairs = 3072;
+void few_pairs_shape(int Q, int64_t pairs, int* g, int* rpl);
 int64_t trace_scratch_words(int Q, int R, int64_t pairs, int shape_g = 0, int shape_rpl = 0);
 // The compiled shapes of the per-pair-length trace pass the autotuner tries
 // for the queries of Q's row class (the exact fit, its default, first);

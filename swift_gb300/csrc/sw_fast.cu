@@ -32,7 +32,7 @@ Shape shape_for(int Q) {
 
 // the compiled (lanes, rows per lane) shapes of the exact passes
 constexpr Shape kShapes[] = {{8, 4}, {4, 8}, {8, 8}, {4, 16}, {8, 13}, {8, 16},
-                             {16, 8}, {16, 13}, {16, 16}, {32, 7}, {32, 10}};
+                             {16, 8}, {16, 13}, {16, 16}, {32, 4}, {32, 7}, {32, 10}};
 constexpr int kNumShapes = (int)(sizeof(kShapes) / sizeof(kShapes[0]));
 // shapes of the per-pair-length trace pass and walk only (swift_sw_pairs'
 // query length classes between the row counts above)
@@ -80,6 +80,7 @@ int launch_shape(cudaStream_t st, const FastArgs& a, int64_t max_pairs) {
   SWIFT_PK(16, 8)
   SWIFT_PK(16, 13)
   SWIFT_PK(16, 16)
+  SWIFT_PK(32, 4)
   SWIFT_PK(32, 7)
   SWIFT_PK(32, 10)
 #undef SWIFT_PK
@@ -108,6 +109,7 @@ int launch_walk(cudaStream_t st, const FastArgs& a, int64_t max_pairs) {
   SWIFT_WK(16, 8)
   SWIFT_WK(16, 13)
   SWIFT_WK(16, 16)
+  SWIFT_WK(32, 4)
   SWIFT_WK(32, 7)
   SWIFT_WK(32, 10)
 #undef SWIFT_WK
@@ -128,6 +130,19 @@ bool fast_params_ok(int Q, int R, int m, int x, int o, int e, int* bias) {
   if (16 * m * Q + b + 16 * (e - o) + 16 >= 0x7C00) return false;
   *bias = b;
   return true;
+}
+
+void few_pairs_shape(int Q, int64_t pairs, int* g, int* rpl) {
+  *g = *rpl = 0;
+  Shape s = {0, 0};
+  if (pairs <= kFewPairs)
+    s = Q <= 128 ? Shape{32, 4} : Q <= 224 ? Shape{32, 7} : Shape{0, 0};
+  else if (pairs <= 2 * kFewPairs && Q > 64 && Q <= 128)
+    s = {16, 8};
+  if (s.G) {
+    *g = s.G;
+    *rpl = s.RPL;
+  }
 }
 
 int64_t trace_scratch_words(int Q, int R, int64_t pairs, int shape_g, int shape_rpl) {
@@ -156,6 +171,7 @@ int packed_shape_candidates(int Q, int32_t* g, int32_t* rpl, int cap) {
   ++n;
   auto add = [&](const Shape& c) {
     const int r = c.G * c.RPL;
+    if (c.G == 32 && c.RPL == 4) return;  // for few pairs only (few_pairs_shape)
     if (r >= rows && r <= rows + rows / 8 + 8 && !(c.G == d.G && c.RPL == d.RPL) && n < cap) {
       g[n] = c.G;
       rpl[n] = c.RPL;

@@ -1848,6 +1848,14 @@ int swift_sw_pairs(swift_ctx* ctx, const char* qry, const int64_t* q_off, const 
         const int tkey = (Q / 8) * 64 + (R + 63) / 64;
         const bool tune = ctx->tuning == 1 && ncand > 1 && !ctx->tuned.count(tkey) &&
                           cnt >= 1024;
+        if (ctx->tuning == 1 && !tune) {
+          auto it = ctx->tuned.find(tkey);
+          if (it != ctx->tuned.end()) {
+            sg = it->second.first;
+            srpl = it->second.second;
+          }
+        }
+        // scratch for the shape that will run, or every one the tuner tries
         int64_t words = 0;
         for (int c = 0; c < (tune ? ncand : 1); ++c)
           words = std::max(words, trace_scratch_words(Q, R, std::min(cnt, sub),
@@ -1874,6 +1882,7 @@ int swift_sw_pairs(swift_ctx* ctx, const char* qry, const int64_t* q_off, const 
         fa.aln = aln;
         fa.best = best2;
         fa.dirs = dirs[0];
+        fa.dirs_words = dirs_words[0];
         fa.qcons = cq;
         fa.rcons = cr;
         fa.cons_stride = cs;
@@ -1915,13 +1924,8 @@ int swift_sw_pairs(swift_ctx* ctx, const char* qry, const int64_t* q_off, const 
             }
           }
           ctx->tuned[tkey] = {cg[best], crpl[best]};
-        }
-        if (ctx->tuning == 1) {
-          auto it = ctx->tuned.find(tkey);
-          if (it != ctx->tuned.end()) {
-            sg = it->second.first;
-            srpl = it->second.second;
-          }
+          sg = cg[best];
+          srpl = crpl[best];
         }
         fa.shape_g = sg;
         fa.shape_rpl = srpl;
@@ -2509,6 +2513,7 @@ static int align_resident_impl(swift_ctx* ctx, const swift_index* idx, const swi
     fa2.list = list;
     fa2.count = count;
     fa2.dirs = dirs;
+    fa2.dirs_words = words;
     if (timed) {
       const size_t need = 2 * (size_t)((n + chunk - 1) / chunk);
       while (ctx->chunk_ev.size() < need) {
@@ -3345,8 +3350,9 @@ static int align_paired_impl(swift_ctx* ctx, const swift_index* idx, const char*
       FastArgs fa2;
       memset(&fa2, 0, sizeof(fa2));
       few_pairs_shape(Q, left_n, &fa2.shape_g, &fa2.shape_rpl);
-      CK(sc.get(&dirs, (size_t)trace_scratch_words(Q, R, std::min<int64_t>(left_n, chunk),
-                                                   fa2.shape_g, fa2.shape_rpl)));
+      fa2.dirs_words = trace_scratch_words(Q, R, std::min<int64_t>(left_n, chunk), fa2.shape_g,
+                                           fa2.shape_rpl);
+      CK(sc.get(&dirs, (size_t)fa2.dirs_words));
       fa2.q = qbuf;
       fa2.w = wbuf;
       fa2.q_stride = qs;

@@ -551,7 +551,8 @@ struct FastArgs {
   const int32_t* r_len;       // (pairs of one launch may differ), or null
   int32_t* ub;                // LCS bound pass: upper bound of the score per pair
   int2* best;                 // trace pass: (score, first maximum cell) per pair
-  uint32_t* dirs;             // trace pass: direction scratch
+  uint32_t* dirs;             // trace pass: direction scratch of dirs_words words
+  int64_t dirs_words;
   int64_t chunk;              // trace pass: pairs of this launch
   char* qcons;                // trace pass: reversed consensus strings
   char* rcons;
@@ -603,7 +604,9 @@ int64_t trace_scratch_words(int Q, int R, int64_t pairs, int shape_g = 0, int sh
 // returns how many.
 int packed_shape_candidates(int Q, int32_t* g, int32_t* rpl, int cap);
 int launch_sw_score(cudaStream_t st, const FastArgs& a, int64_t max_pairs);
-// before / after (optional) are recorded around the trace pass alone
+// before / after (optional) are recorded around the trace pass alone; 0 when
+// nothing could be launched, also when a.dirs is too small for max_pairs in
+// the shape the launch takes (trace_scratch_words)
 int launch_sw_trace(cudaStream_t st, const FastArgs& a, int64_t max_pairs,
                     cudaEvent_t before = nullptr, cudaEvent_t after = nullptr);
 // sw_lcs.cu: a.ub[p] = match * LCS(query, window) for the listed pairs, and

@@ -192,6 +192,7 @@ int launch_sw_trace(cudaStream_t st, const FastArgs& a, int64_t max_pairs, cudaE
                     cudaEvent_t after) {
   // the walk stores 32-bit words, and reads words of the query and window rows
   if (a.cons_stride % 4 != 0 || (a.q_stride | a.w_stride) % 4 != 0) return 0;
+  if (trace_scratch_words(a.Q, a.R, max_pairs, a.shape_g, a.shape_rpl) > a.dirs_words) return 0;
   FastArgs b = a;
   b.chunk = max_pairs;
   b.one = 1;

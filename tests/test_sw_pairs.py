@@ -249,3 +249,26 @@ def test_long_workload_vs_oracle(ctx, oracle):
     ws = [ref[a:a + b] for a, b in zip(ro, rl)]
     check_against_oracle(res, qs, ws, oracle, (2, -1, -10, -1))
     assert (res["score"] > 1000).all()  # every query aligns across its region
+
+
+@pytest.mark.parametrize("q", [96, 120, 250])
+def test_second_call_with_a_tuned_shape(ctx, sg, q):
+    # the direction scratch is sized for the shape that runs, also where the
+    # tuned shape (whatever it is) needs more than the default one: a launch
+    # with too little scratch is refused, so the calls succeed and agree
+    rng = np.random.default_rng(q)
+    n, r = 3000, q + 128
+    ref = np.frombuffer(b"ACGT", np.uint8)[rng.integers(0, 4, 400_000)].tobytes()
+    ro = rng.integers(0, 400_000 - r, n)
+    qo = ro + rng.integers(0, 128, n)
+    ql, rl = np.full(n, q, np.int32), np.full(n, r, np.int32)
+    c = sg.Context(0)
+    try:
+        first, st = c.sw_pairs(ref, qo, ql, ref, ro, rl)
+        again, st2 = c.sw_pairs(ref, qo, ql, ref, ro, rl)
+    finally:
+        c.close()
+    assert st["tune_ms"] > 0 and st2["tune_ms"] == 0
+    for key in ("score", "start", "end", "len"):
+        assert np.array_equal(first[key], again[key]), key
+    assert (first["score"] == 2 * q).all()

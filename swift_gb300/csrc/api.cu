@@ -405,6 +405,16 @@ __global__ void aln_to_ref_layout_kernel(const DevAln* __restrict__ aln, int64_t
 // costs less than the passes, lists and host round trips that would spare
 // most of them: at these sizes each pass lasts as long as one pair does.
 constexpr int64_t kDirectPairs = 3072;
+// At most this many pairs all run on the int32 kernel: its warp a pair holds
+// directions in shared memory and walks them there, so at 1,024 pairs it ends
+// before the packed trace pass and walk, two launches of a few warps (100 x
+// 300: 92 against 121 us; at 2,048 143 each).
+constexpr int64_t kFewGeneric = 1024;
+// swift_sw_batch: from here on (pairs, and query rows in all) the packed
+// passes are faster (2,048 pairs of 36 x 100: 66 us on the int32 kernel, 77
+// packed; 4,096: 92 each; 2,048 of 100 x 300: 143 each; 2,048 of 250 x 500:
+// 511 against 306; 1,024 of 250 x 500: 271 against 290).
+constexpr int64_t kBatchPackedPairs = 2048, kBatchPackedRows = 200000;
 
 struct SeedOut {
   int32_t *m_read = nullptr, *m_strand = nullptr, *m_ri = nullptr, *m_sh = nullptr,
@@ -1415,12 +1425,18 @@ int swift_sw_batch(swift_ctx* ctx, const char* qry, const char* ref, int32_t Q, 
     CK(cudaMemcpyAsync(t, ref, (size_t)n * (R + 1), cudaMemcpyHostToDevice, st));
     dw = t;
   }
-  DevAln* aln;
-  CK(sc.get(&aln, (size_t)n));
   const bool out_dev = is_dev(score);
   char *dqc = qcons, *drc = rcons;
   if (!is_dev(qcons)) CK(sc.get(&dqc, (size_t)n * cs));
   if (!is_dev(rcons)) CK(sc.get(&drc, (size_t)n * cs));
+  float* dscore = score;
+  int32_t *dstart = start, *dend = end, *dlen = len;
+  if (!out_dev) {
+    CK(sc.get(&dscore, n));
+    CK(sc.get(&dstart, n));
+    CK(sc.get(&dend, n));
+    CK(sc.get(&dlen, n));
+  }
   SwArgs a;
   memset(&a, 0, sizeof(a));
   a.q = dq;
@@ -1433,25 +1449,117 @@ int swift_sw_batch(swift_ctx* ctx, const char* qry, const char* ref, int32_t Q, 
   a.mismatch = x;
   a.gap_open = o;
   a.gap_ext = e;
-  a.n = n;
-  a.aln = aln;
   a.qcons = dqc;
   a.rcons = drc;
   a.cons_stride = cs;
-  int rc = launch_sw(st, a, &ctx->err);
-  if (rc != SWIFT_OK) return rc;
-  CKLAUNCH();
-  float* dscore = score;
-  int32_t *dstart = start, *dend = end, *dlen = len;
-  if (!out_dev) {
-    CK(sc.get(&dscore, n));
-    CK(sc.get(&dstart, n));
-    CK(sc.get(&dend, n));
-    CK(sc.get(&dlen, n));
+  // From kBatchPackedPairs and -Rows on, pairs of bases run on the packed trace
+  // pass and walk, in chunks that bound its scratch; the others, and every
+  // pair where the scoring or that scratch is not to be had, on the int32
+  // kernel, which needs none.
+  int bias = 0;
+  bool packed = n >= kBatchPackedPairs && n * Q >= kBatchPackedRows &&
+                fast_params_ok(Q, R, m, x, o, e, &bias);
+  const int64_t chunk = std::min<int64_t>(n, 131072);
+  BatchArgs ba;
+  FastArgs fa;
+  BatchOutArgs bo;
+  int32_t* counts = nullptr;
+  memset(&ba, 0, sizeof(ba));
+  memset(&fa, 0, sizeof(fa));
+  memset(&bo, 0, sizeof(bo));
+  if (packed) {
+    ba.Q = Q;
+    ba.R = R;
+    ba.q_stride = ((int64_t)Q + 16) & ~(int64_t)15;
+    ba.w_stride = ((int64_t)R + 16) & ~(int64_t)15;
+    fa.cons_stride = (cs + 15) & ~(int64_t)15;  // the walk stores words
+    few_pairs_shape(Q, chunk, &fa.shape_g, &fa.shape_rpl);
+    fa.dirs_words = trace_scratch_words(Q, R, chunk, fa.shape_g, fa.shape_rpl);
+    packed = sc.get(&ba.qbuf, (size_t)(chunk * ba.q_stride)) == cudaSuccess &&
+             sc.get(&ba.wbuf, (size_t)(chunk * ba.w_stride)) == cudaSuccess &&
+             sc.get(&ba.fast, (size_t)chunk) == cudaSuccess &&
+             sc.get(&ba.gen, (size_t)chunk) == cudaSuccess &&
+             sc.get(&ba.packed, (size_t)chunk) == cudaSuccess &&
+             sc.get(&counts, 2) == cudaSuccess &&
+             sc.get(&fa.best, (size_t)chunk) == cudaSuccess &&
+             sc.get(&fa.qcons, (size_t)(chunk * fa.cons_stride)) == cudaSuccess &&
+             sc.get(&fa.rcons, (size_t)(chunk * fa.cons_stride)) == cudaSuccess &&
+             sc.get(&fa.dirs, (size_t)fa.dirs_words) == cudaSuccess;
+    if (!packed) cudaGetLastError();  // no memory for it: the int32 kernel
   }
-  aln_to_ref_layout_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(aln, n, dscore, dstart, dend,
-                                                                       dlen);
-  CKLAUNCH();
+  DevAln* aln;
+  CK(sc.get(&aln, (size_t)(packed ? chunk : n)));
+  if (!packed) {
+    a.n = n;
+    a.aln = aln;
+    int rc = launch_sw(st, a, &ctx->err);
+    if (rc != SWIFT_OK) return rc;
+    CKLAUNCH();
+    aln_to_ref_layout_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(aln, n, dscore, dstart,
+                                                                         dend, dlen);
+    CKLAUNCH();
+  }
+  for (int64_t c0 = 0; packed && c0 < n; c0 += chunk) {
+    const int64_t cn = std::min(chunk, n - c0);
+    ba.q = dq + c0 * (Q + 1);
+    ba.w = dw + c0 * (R + 1);
+    ba.n = cn;
+    ba.n_fast = counts;
+    ba.n_gen = counts + 1;
+    CK(cudaMemsetAsync(counts, 0, 2 * sizeof(int32_t), st));
+    launch_pack_batch(st, ba);
+    CKLAUNCH();
+    a.q = ba.q;
+    a.w = ba.w;
+    a.n = cn;
+    a.aln = aln;
+    a.qcons = dqc + c0 * cs;
+    a.rcons = drc + c0 * cs;
+    a.list = ba.gen;
+    a.count = ba.n_gen;
+    // the int32 kernel's few pairs beside the trace pass (as in the aligner)
+    SideJoin generic(ctx);
+    int rc = side_fork(ctx);
+    if (rc != SWIFT_OK) return rc;
+    generic.armed = true;
+    rc = launch_sw(ctx->side, a, &ctx->err);
+    if (rc != SWIFT_OK) return rc;
+    CKLAUNCH();
+    fa.q = ba.qbuf;
+    fa.w = ba.wbuf;
+    fa.q_stride = ba.q_stride;
+    fa.w_stride = ba.w_stride;
+    fa.Q = Q;
+    fa.R = R;
+    fa.match = m;
+    fa.mismatch = x;
+    fa.gap_open = o;
+    fa.gap_ext = e;
+    fa.bias = bias;
+    fa.aln = aln;
+    fa.list = ba.fast;
+    fa.count = ba.n_fast;
+    if (launch_sw_trace(st, fa, cn) == 0)
+      return fail(ctx, SWIFT_E_DEVICE, "trace pass could not launch");
+    CKLAUNCH();
+    rc = generic.join();
+    if (rc != SWIFT_OK) return rc;
+    bo.n = cn;
+    bo.aln = aln;
+    bo.packed = ba.packed;
+    bo.score = dscore + c0;
+    bo.start = dstart + c0;
+    bo.end = dend + c0;
+    bo.len = dlen + c0;
+    bo.qfrom = fa.qcons;
+    bo.rfrom = fa.rcons;
+    bo.from_stride = fa.cons_stride;
+    bo.qto = a.qcons;
+    bo.rto = a.rcons;
+    bo.to_stride = cs;
+    launch_batch_out(st, bo);
+    CKLAUNCH();
+  }
   if (!out_dev) {
     CK(cudaMemcpyAsync(score, dscore, n * 4, cudaMemcpyDeviceToHost, st));
     CK(cudaMemcpyAsync(start, dstart, n * 4, cudaMemcpyDeviceToHost, st));
@@ -2195,7 +2303,7 @@ static int align_resident_impl(swift_ctx* ctx, const swift_index* idx, const swi
     }
   }
   int bias = 0;
-  const bool fast_ok =
+  bool fast_ok =
       ctx->sw_path != 1 && fast_params_ok(Q, kWin, p->match, p->mismatch, p->gap_open, p->gap_ext, &bias);
   // SAM output prints every record: no selection, every pair traced
   const bool sam = p->out_format == 1;
@@ -2321,6 +2429,8 @@ static int align_resident_impl(swift_ctx* ctx, const swift_index* idx, const swi
     }
   }
   // few records: each traced at once (see kDirectPairs); else bounded selection
+  // (below kFewGeneric on the int32 kernel alone)
+  if (ctx->sw_path == 0 && n <= kFewGeneric) fast_ok = false;
   const bool direct = fast_ok && ctx->sw_path == 0 && !sam && n <= kDirectPairs;
   const bool bounded = fast_ok && ctx->sw_path == 0 && !sam && !direct;
   const int Qs = (Q + 16) & ~15;
@@ -2665,7 +2775,7 @@ static int align_resident_impl(swift_ctx* ctx, const swift_index* idx, const swi
         pairs, keep, cand, n, fast_ok && !direct ? 0 : 1, list2, cnt + 4, cnt + 5);
     CKLAUNCH();
     ++launches;
-    if (!direct) {
+    if (fast_ok && !direct) {
       CK(rb.get(h_cnt, cnt, sizeof(h_cnt)));
       CK(rb.sync());
       rc = trace_list(list2, cnt + 4, h_cnt[4], false);
@@ -3115,7 +3225,7 @@ static int align_paired_impl(swift_ctx* ctx, const swift_index* idx, const char*
   }
   const bool sam = p->out_format == 1;
   int bias = 0;
-  const bool fast_ok = fast_params_ok(Q, R, p->match, p->mismatch, p->gap_open, p->gap_ext, &bias);
+  bool fast_ok = fast_params_ok(Q, R, p->match, p->mismatch, p->gap_open, p->gap_ext, &bias);
   // Gapless pass over every record (ungapped.cu): `all` is the output's view
   ReadPackArgs rp;
   memset(&rp, 0, sizeof(rp));
@@ -3304,6 +3414,8 @@ static int align_paired_impl(swift_ctx* ctx, const swift_index* idx, const char*
   pl.wbuf = wbuf;
   pl.q_stride = qs;
   pl.w_stride = ws;
+  // few records left: all on the int32 kernel (kFewGeneric)
+  if (left_n <= kFewGeneric) fast_ok = false;
   launch_pe_pairs(st, pl);
   CKLAUNCH();
   launches += left_n > 0 ? 1 : 0;

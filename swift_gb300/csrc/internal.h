@@ -462,6 +462,35 @@ constexpr int64_t kStaticSwPairs = SWIFT_SW_NOALLOC_MAX_PAIRS;
 int static_sw_scratch(int device, DevAln** out, std::string* err);
 int launch_sw(cudaStream_t st, const SwArgs& a, std::string* err);
 
+// batch.cu: swift_sw_batch's pairs on the packed passes
+struct BatchArgs {
+  const char* q;              // query i at q + i * (Q + 1), window i at w + i * (R + 1)
+  const char* w;
+  int Q, R;
+  int64_t n;
+  char* qbuf;                 // out: rows of q_stride and w_stride bytes (multiples of
+  char* wbuf;                 // 16), zero past Q and R
+  int64_t q_stride, w_stride;
+  int32_t *fast, *n_fast;     // out: pairs of A, C, G, T bytes (either case) only,
+  int32_t *gen, *n_gen;       // and the others
+  uint8_t* packed;            // out, per pair: 1 in the fast list
+};
+void launch_pack_batch(cudaStream_t st, const BatchArgs& a);
+// results in the caller's layout; the strings (stride to_stride, any
+// alignment) copied from from_stride rows where packed is set
+struct BatchOutArgs {
+  int64_t n;
+  const DevAln* aln;
+  const uint8_t* packed;
+  float* score;
+  int32_t *start, *end, *len;
+  const char *qfrom, *rfrom;
+  int64_t from_stride;
+  char *qto, *rto;
+  int64_t to_stride;
+};
+void launch_batch_out(cudaStream_t st, const BatchOutArgs& a);
+
 // pairs_var.cu: explicit pairs of varying lengths, sorted by shape
 constexpr uint32_t kVarKeys = 1u << 21;  // shape keys: generic bit, Q (9 bits), R (11 bits)
 // the top eight keys: long pairs (sw_long.cu) by rows-per-lane class (key

@@ -16,7 +16,7 @@
 // stage, so every value is written before it is read and a ring of 128
 // columns is never overrun.  Each thread streams its 2-bit direction codes
 // per wavefront step to global scratch (four steps per 16-byte store);
-// sw_long_walk_kernel then walks the reference's traceback, one thread per
+// sw_long_walk_kernel then walks the reference's traceback, one warp per
 // pair, carrying the cell score to tell NONE from LEFT.
 #include <type_traits>
 
@@ -257,12 +257,34 @@ __global__ void __launch_bounds__(kLT, 2) sw_long_kernel(LongArgs a) {
   }
 }
 
-// Traceback walk over the long kernel's direction codes, one thread per
-// pair (the same rules as sw_walk_kernel).
+// Traceback walk over the long kernel's direction codes (the same rules as
+// sw_walk_kernel), one warp per pair.
+//
+// A walk is a chain of dependent reads.  The warp fetches a tile of 256
+// direction words at once: of the threads whose rows the walk passes next,
+// the steps around the diagonal from its cell (plus the query and window
+// bytes there); the moves then run from shared memory, every lane alike,
+// until one leaves the tile.  (One thread per pair read four words at a time,
+// and some walk of its warp waited for memory on almost every move: 4.2 ms
+// for queries of 3 to 4 kb, 0.95 ms now.)
+constexpr int kTileWords = 256;
+constexpr int kTileBytes = 256;  // of query and of window, before the cell
+constexpr int kWalkWarps = 4;
+
 template <int RPL>
-__global__ void __launch_bounds__(128) sw_long_walk_kernel(LongArgs a) {
-  const int64_t item = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (item >= a.n) return;
+__global__ void __launch_bounds__(kWalkWarps * 32) sw_long_walk_kernel(LongArgs a) {
+  // words per stream: the columns a diagonal crosses in RPL rows, 9 before
+  // them and about 5 past (gaps)
+  constexpr int kWords = RPL <= 4 ? 16 : 32, kStreams = kTileWords / kWords;
+  __shared__ __align__(16) uint32_t tile_all[kWalkWarps][kTileWords];
+  __shared__ char q_all[kWalkWarps][kTileBytes], w_all[kWalkWarps][kTileBytes];
+  __shared__ int lo_all[kWalkWarps][kStreams];
+  const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int64_t item = (int64_t)blockIdx.x * kWalkWarps + wib;
+  if (item >= a.n) return;  // (no block-wide synchronisation below)
+  uint32_t* tile = tile_all[wib];
+  char *qs = q_all[wib], *ws = w_all[wib];
+  int* lo = lo_all[wib];  // per stream: its first step in the tile
   const int32_t p = a.list[item];
   const int R = a.r_len[p];
   const char* qg = a.qry + a.q_off[p];
@@ -270,20 +292,42 @@ __global__ void __launch_bounds__(128) sw_long_walk_kernel(LongArgs a) {
   const int S4 = (R + 31 + 3) & ~3;
   const uint32_t* dirs = a.dirs + a.dir_off[item];
   const int W = R + 1;
-  // four consecutive steps of one thread per load: a diagonal run of the
-  // walk stays in one thread's rows and moves one step back per cell
-  int64_t last = -1;
-  uint4 words = make_uint4(0, 0, 0, 0);
-  auto code_at = [&](int i, int jj) -> uint32_t {
-    const int t = (i - 1) / RPL, k = (i - 1) % RPL, ln = t & 31;
-    const int64_t at = (int64_t)t * S4 + (jj + ln - 1);
-    if ((at & ~(int64_t)3) != last) {
-      last = at & ~(int64_t)3;
-      words = __ldcg(reinterpret_cast<const uint4*>(dirs + last));
+  int t0 = -1, rows0 = 0, cols0 = 0;  // the tile's first thread; bytes before row / column
+  auto fetch = [&](int i, int jj) {  // the tile from cell (i, jj) on
+    t0 = (i - 1) / RPL;
+    rows0 = i;
+    cols0 = jj;
+    const int k0 = (i - 1) - t0 * RPL;
+    __syncwarp();
+#pragma unroll
+    for (int v = 0; v < kTileWords / 128; ++v) {
+      const int at = (v * 32 + lane) * 4, m = at / kWords, t = t0 - m;
+      // the column at which a diagonal enters thread t's rows, as its step
+      const int enter = jj - (m == 0 ? 0 : k0 + 1 + (m - 1) * RPL) + (t & 31) - 1;
+      const int first = max((enter + 8 - (kWords - 1)) & ~3, 0);
+      const int s = first + (at & (kWords - 1));
+      uint4 x = make_uint4(0, 0, 0, 0);
+      if (t >= 0 && s + 4 <= S4)
+        x = __ldcg(reinterpret_cast<const uint4*>(dirs + (int64_t)t * S4 + s));
+      *reinterpret_cast<uint4*>(tile + at) = x;
+      if ((at & (kWords - 1)) == 0) lo[m] = first;
     }
-    const int q = (int)(at & 3);
-    const uint32_t word = q == 0 ? words.x : q == 1 ? words.y : q == 2 ? words.z : words.w;
-    return (word >> (2 * k)) & 3u;
+    for (int b = lane; b < kTileBytes; b += 32) {
+      if (b < i) qs[b] = qg[i - 1 - b];
+      if (b < jj) ws[b] = wg[jj - 1 - b];
+    }
+    __syncwarp();
+  };
+  // the code of cell (i, jj); fetches a tile when it is not in this one
+  auto code_at = [&](int i, int jj) -> uint32_t {
+    const int t = (i - 1) / RPL, k = (i - 1) - t * RPL, step = jj + (t & 31) - 1;
+    int m = t0 - t;
+    if (t0 < 0 || m >= kStreams || step < lo[m] || step >= lo[m] + kWords ||
+        rows0 - i >= kTileBytes - 1 || cols0 - jj >= kTileBytes - 1) {
+      fetch(i, jj);
+      m = 0;
+    }
+    return (tile[m * kWords + (step - lo[m])] >> (2 * k)) & 3u;
   };
   enum : int { kNone = 0, kDiag = 1, kUp = 2, kLeft = 3 };
   auto dir_of = [](uint32_t code, int h) -> int {
@@ -296,56 +340,47 @@ __global__ void __launch_bounds__(128) sw_long_walk_kernel(LongArgs a) {
   int cr = b.y / W, cc = b.y % W;
   int h = b.x;
   int d = (cr == 0 || cc == 0) ? kNone : dir_of(code_at(cr, cc), h);
-  int nr = cr, nc = cc, nh = h, nd = kNone;
-  auto advance = [&]() {
-    nr = cr - ((d == kDiag || d == kUp) ? 1 : 0);
-    nc = cc - ((d == kDiag || d == kLeft) ? 1 : 0);
-    if (d == kNone) {
-      nh = h;
-      nd = kNone;
-      return;
+  int tick = -1, nref = -1, start = 0;
+  char my_q = 0, my_r = 0;  // the bytes of move tick with tick % 32 == lane
+  while (d != kNone) {
+    const bool up = d != kLeft, left = d != kUp;  // row / column move
+    const char qb = qs[rows0 - cr], rb = ws[cols0 - cc];
+    ++tick;
+    nref += left ? 1 : 0;
+    if (lane == (tick & 31)) {
+      my_r = left ? rb : '-';
+      my_q = up ? qb : '-';
     }
-    const uint32_t pc = (nr == 0 || nc == 0) ? 0u : code_at(nr, nc);
+    if ((tick & 31) == 31 && qc) {
+      rc[tick - 31 + lane] = my_r;
+      qc[tick - 31 + lane] = my_q;
+    }
+    start = cc;
+    cr -= up ? 1 : 0;
+    cc -= left ? 1 : 0;
+    if (cr == 0 || cc == 0) break;
+    const uint32_t pc = code_at(cr, cc);
     if (d == kDiag) {
-      const int qb = upcase((uint8_t)qg[cr - 1]), rb = upcase((uint8_t)wg[cc - 1]);
-      nh = h - ((qb == rb || qb == 'N' || rb == 'N') ? m : x);
+      const int uq = upcase((uint8_t)qb), ur = upcase((uint8_t)rb);
+      h -= (uq == ur || uq == 'N' || ur == 'N') ? m : x;
     } else {
       // the gap costs gap_ext when the predecessor itself moved the same way
-      const bool same = nr != 0 && nc != 0 && (d == kUp ? pc == 1u : pc == 0u);
-      nh = h - (same ? e : o);
+      h -= (d == kUp ? pc == 1u : pc == 0u) ? e : o;
     }
-    nd = (nr == 0 || nc == 0) ? kNone : dir_of(pc, nh);
-  };
-  advance();
-  int tick = -1, nref = -1, start = 0;
-  auto emit = [&](char r, char q) {
-    ++tick;
-    if (qc) {
-      rc[tick] = r;
-      qc[tick] = q;
-    }
-  };
-  while ((cr != nr || cc != nc) && nc != 0 && nr != 0) {
-    char rch = '-';
-    if (nc != cc) { rch = wg[cc - 1]; ++nref; }
-    emit(rch, nr == cr ? '-' : qg[cr - 1]);
-    start = cc;
-    cr = nr; cc = nc; h = nh; d = nd;
-    if (d == kNone) break;
-    advance();
+    d = dir_of(pc, h);
   }
-  if ((cr != nr || cc != nc) && (nc == 0 || nr == 0)) {
-    char rch = '-';
-    if (nc != cc) { rch = wg[cc - 1]; ++nref; }
-    emit(rch, nr == cr ? '-' : qg[cr - 1]);
-    start = cc;
+  if (qc && tick >= 0 && lane <= (tick & 31) && (tick & 31) != 31) {
+    rc[(tick & ~31) + lane] = my_r;
+    qc[(tick & ~31) + lane] = my_q;
   }
-  DevAln out;
-  out.score = b.x;
-  out.start = start;
-  out.end = start + nref;
-  out.len = tick + 1;
-  a.aln[p] = out;
+  if (lane == 0) {
+    DevAln out;
+    out.score = b.x;
+    out.start = start;
+    out.end = start + nref;
+    out.len = tick + 1;
+    a.aln[p] = out;
+  }
 }
 
 template <int RPL>
@@ -355,7 +390,8 @@ int launch_long_rpl(cudaStream_t st, const LongArgs& a, bool prof) {
     sw_long_kernel<RPL, true><<<(unsigned)a.n, kLT, smem, st>>>(a);
   else
     sw_long_kernel<RPL, false><<<(unsigned)a.n, kLT, smem, st>>>(a);
-  sw_long_walk_kernel<RPL><<<(unsigned)((a.n + 127) / 128), 128, 0, st>>>(a);
+  sw_long_walk_kernel<RPL><<<(unsigned)((a.n + kWalkWarps - 1) / kWalkWarps), kWalkWarps * 32, 0,
+                             st>>>(a);
   return 2;
 }
 

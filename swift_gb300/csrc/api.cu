@@ -1810,6 +1810,7 @@ int swift_sw_pairs(swift_ctx* ctx, const char* qry, const int64_t* q_off, const 
     va.q_stride = q_stride;
     va.w_stride = w_stride;
     va.long_prof = long_prof_ok(m, x, o, kLongMaxQ);
+    va.long16_max_q = long16_max_q(m, x, o, e);
     va.class_ok = 0;
     for (int c = 0; mode == 0 && c < 6; ++c)
       if (fast_params_ok(packed_class_max_q(c), kFastMaxR, m, x, o, e, &bias0)) va.class_ok |= 1u << c;
@@ -1884,7 +1885,7 @@ int swift_sw_pairs(swift_ctx* ctx, const char* qry, const int64_t* q_off, const 
       for (uint32_t s = 0; s < nseg; ++s) {
         if ((uint32_t)hk[s] >= kVarLongKey) {
           long_groups.push_back({hs[s], hc[s]});
-          long_class.push_back((int)((uint32_t)hk[s] - kVarLongKey));  // 2 class + profile bit
+          long_class.push_back((int)((uint32_t)hk[s] - kVarLongKey));  // 4 class + kernel
           continue;
         }
         const bool gen = (hk[s] >> 20) & 1;
@@ -2076,8 +2077,7 @@ int swift_sw_pairs(swift_ctx* ctx, const char* qry, const int64_t* q_off, const 
         }
         CK(cudaStreamSynchronize(st));
         struct LongBatch {
-          int rpl;
-          bool prof;
+          int rpl, kind;
           int64_t b0, nb, words;
         };
         std::vector<LongBatch> batches;
@@ -2092,8 +2092,7 @@ int swift_sw_pairs(swift_ctx* ctx, const char* qry, const int64_t* q_off, const 
             const int64_t cu = (int64_t)hql[u] * hrl[u], cv = (int64_t)hql[v] * hrl[v];
             return cu != cv ? cu > cv : u < v;
           });
-          const int rpl = 4 * ((long_class[lg] >> 1) + 1);
-          const bool prof = long_class[lg] & 1;
+          const int rpl = 4 * ((long_class[lg] >> 2) + 1), kind = long_class[lg] & 3;
           int64_t b0 = 0;
           while (b0 < cnt) {
             int64_t words = 0, b1 = b0;
@@ -2102,7 +2101,7 @@ int swift_sw_pairs(swift_ctx* ctx, const char* qry, const int64_t* q_off, const 
               words += long_slot_words(hrl[g[b1]]);
               ++b1;
             }
-            batches.push_back({rpl, prof, at + b0, b1 - b0, words});
+            batches.push_back({rpl, kind, at + b0, b1 - b0, words});
             max_words = std::max(max_words, words);
             b0 = b1;
           }
@@ -2116,6 +2115,10 @@ int swift_sw_pairs(swift_ctx* ctx, const char* qry, const int64_t* q_off, const 
         CK(cudaMemcpyAsync(dlist, ids.data(), n_long * 4, cudaMemcpyHostToDevice, st));
         CK(cudaMemcpyAsync(doff, off.data(), n_long * 8, cudaMemcpyHostToDevice, st));
         const int n_regions = batches.size() > 1 ? 2 : 1;
+        // whole GiB, so that calls of like sizes find the pool's block again
+        // (a new size maps memory anew, 1.3 ms at 4 GB)
+        constexpr int64_t kGiB = 1 << 28;
+        if (max_words > kGiB) max_words = (max_words + kGiB - 1) & ~(kGiB - 1);
         for (int r = 0; r < n_regions; ++r) {
           if (max_words > dirs_words[r]) {
             CK(sc.get(&dirs[r], (size_t)max_words));
@@ -2145,7 +2148,6 @@ int swift_sw_pairs(swift_ctx* ctx, const char* qry, const int64_t* q_off, const 
           la.mismatch = x;
           la.gap_open = o;
           la.gap_ext = e;
-          la.bias = long_bias(o);
           la.dirs = dirs[b & 1];
           la.dir_off = doff + lb.b0;
           la.best = best2;
@@ -2153,7 +2155,7 @@ int swift_sw_pairs(swift_ctx* ctx, const char* qry, const int64_t* q_off, const 
           la.qcons = cq;
           la.rcons = cr;
           la.cons_stride = cs;
-          const int kk = launch_sw_long(bs, la, lb.rpl, lb.prof);
+          const int kk = launch_sw_long(bs, la, lb.rpl, lb.kind);
           if (kk == 0) return fail(ctx, SWIFT_E_DEVICE, "long pass could not launch");
           launches += kk;
           CKLAUNCH();

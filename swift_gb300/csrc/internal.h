@@ -493,9 +493,14 @@ void launch_batch_out(cudaStream_t st, const BatchOutArgs& a);
 
 // pairs_var.cu: explicit pairs of varying lengths, sorted by shape
 constexpr uint32_t kVarKeys = 1u << 21;  // shape keys: generic bit, Q (9 bits), R (11 bits)
-// the top eight keys: long pairs (sw_long.cu) by rows-per-lane class (key
-// bits 2-1) and whether they hold only ACGTN bytes (bit 0)
-constexpr uint32_t kVarLongKey = kVarKeys - 8;
+// the top sixteen keys: long pairs (sw_long.cu) by rows-per-thread class (key
+// bits 3-2) and kernel (bits 1-0)
+constexpr uint32_t kVarLongKey = kVarKeys - 16;
+enum : int {
+  kLongBytes = 0,  // any bytes
+  kLongProf = 1,   // A, C, G, T, N (either case) only
+  kLong16 = 2,     // A, C, G, T only, and cells that fit 16 bits
+};
 // pairs beyond the warp-per-pair kernels' shapes go to the long kernel
 __host__ __device__ inline bool var_pair_long(int Q, int R) {
   return Q > 256 || R > 1024 || (Q > 128 && R > 768);
@@ -513,6 +518,7 @@ struct VarPairArgs {
   int64_t q_stride, w_stride;
   uint32_t class_ok;          // bit c: the packed passes take this scoring for class c
   bool long_prof;             // the long kernel's profile path takes this scoring
+  int long16_max_q;           // the longest query its 16-bit form takes (0: none)
   int fast_max_r;
   uint32_t* key;              // per pair
   uint32_t* hist;             // per key
@@ -541,7 +547,9 @@ struct LongArgs {
   const int32_t* list;        // pair ids of this launch
   int64_t n;
   int max_r;                  // longest window of the launch
-  int match, mismatch, gap_open, gap_ext, bias;
+  int match, mismatch, gap_open, gap_ext;
+  int bias;                   // set by launch_sw_long, with
+  uint32_t one, four;         // 1 and 4 as values the compiler cannot fold
   uint32_t* dirs;             // direction scratch: the slot of item i at dirs + dir_off[i],
   const int64_t* dir_off;     // long_slot_words(R of its pair) words
   int2* best;                 // per pair: (score, first maximum cell)
@@ -552,13 +560,13 @@ struct LongArgs {
 };
 int long_rows_per_lane(int Q);           // 4, 8, 12 or 16; 0 beyond 4096
 int64_t long_slot_words(int R);          // direction words of one pair (16-byte multiple)
-// the long kernel's cell bias for a gap-open penalty, and whether its
-// profile path takes a scoring for queries up to max_q rows; prof: every
-// pair of the launch holds only ACGTN bytes (either case) and
-// long_prof_ok(...) holds
-int long_bias(int gap_open);
+// whether the long kernel's profile path (kLongProf) takes a scoring for
+// queries up to max_q rows, and the longest query its 16-bit form (kLong16)
+// takes
 bool long_prof_ok(int m, int x, int gap_open, int max_q);
-int launch_sw_long(cudaStream_t st, const LongArgs& a, int rpl, bool prof);
+int long16_max_q(int m, int x, int o, int e);
+// kind: kLongBytes, kLongProf or kLong16, of every pair of the launch
+int launch_sw_long(cudaStream_t st, const LongArgs& a, int rpl, int kind);
 
 // sw_fast.cu: packed 16-bit passes (score of every pair; trace of printed pairs)
 // Suffix LCS values: window columns per block (the wavefront steps between

@@ -18,6 +18,9 @@
 // per wavefront step to global scratch (four steps per 16-byte store);
 // sw_long_walk_kernel then walks the reference's traceback, one warp per
 // pair, carrying the cell score to tell NONE from LEFT.
+//
+// Pairs of A, C, G and T only whose scores fit run sw_long16_kernel below,
+// two query strips per thread in 16-bit halves.
 #include <type_traits>
 
 #include "internal.h"
@@ -257,7 +260,280 @@ __global__ void __launch_bounds__(kLT, 2) sw_long_kernel(LongArgs a) {
   }
 }
 
-// Traceback walk over the long kernel's direction codes (the same rules as
+// The same recurrence in packed 16-bit halves, for pairs of A, C, G, T bytes
+// (either case) with 4 * match * Q + bias below 2^15 (long16_max_q).
+//
+// Cells are 4 * H + code + B with code 3 DIAG or NONE, 2 UP, 1 LEFT: one
+// three-way maximum gives H and the direction (on equal H DIAG before UP
+// before LEFT; DIAG and NONE need no telling apart, a cell is NONE exactly
+// when H = 0), and a cleared code bit selects the next cells' gap penalties.
+//
+// Layout.  Thread t owns two strips of RH query rows, virtual lane 2 t in the
+// low half and 2 t + 1, the next RH rows, in the high half, one window column
+// behind: the warp is a wavefront of 64 strips.  The low strip's bottom row
+// moves to the high half of the next step by one funnel shift, which also
+// brings in the lane above's high strip (one shuffle).  The window selector
+// of a column holds the low half's base and, a column back, the high half's.
+// Steps in which some lane's column lies outside the window score mismatches
+// there: cells left of the window then keep H = 0, and cells right of it stay
+// below the window's maximum.  Warps follow one another 5 stages of 16 steps
+// apart (a strip's bottom row leaves the warp 62 steps after it enters), over
+// rings of 64 columns.
+//
+// First maximum.  A lane only keeps the maximum of its cells over 4 steps;
+// where it reaches the warp's largest so far, which happens while the
+// alignment itself passes and rarely else, it puts those steps' cells aside
+// and goes on; only the last ones put aside, and equal maxima, are looked
+// through cell by cell.  (Looking at once made every warp of the CTA wait for
+// the one the alignment passes: 3.7 ms for queries of 3 to 4 kb, whose
+// barriers took half of it, against 3.5 ms for pairs of all sizes.)  A cell of the
+// final maximum is never missed, since the warp's largest so far never
+// exceeds it.
+//
+// Per two cells 12.5 instructions, 6.5 on the ALU pipe, where the int32
+// kernel takes 28 and 18 (500 pairs of 1-4 kb by 2-8 kb: 3.5 ms, 13.4 before
+// over four launches).
+constexpr int kStage16 = 16;
+constexpr int kLag16 = 5;    // stages between neighbouring warps
+constexpr int kRing16 = 64;  // ring columns
+constexpr int kPad16 = 64;   // selectors before column 0
+constexpr int kSel16 = kPad16 + 96;  // and in all beside the window's columns
+
+template <int RH>
+__device__ __forceinline__ void long16_pair(const LongArgs& a, const int64_t item, const int32_t p,
+                                            const int Q, const int R, uint8_t* smem) {
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const char* qg = a.qry + a.q_off[p];
+  const char* wg = a.ref + a.r_off[p];
+  uint16_t* wsel = reinterpret_cast<uint16_t*>(smem);  // [kPad16 + column]
+  uint32_t* ring = reinterpret_cast<uint32_t*>(smem + ((2 * (a.max_r + kSel16) + 15) & ~15));
+  for (int c = tid; c < R + kSel16; c += kLT) {
+    const int j = c - kPad16;
+    const uint32_t lo = j >= 1 && j <= R ? (uint32_t)class5((uint8_t)wg[j - 1]) : 0u;
+    const uint32_t hi = j >= 2 && j <= R + 1 ? (uint32_t)class5((uint8_t)wg[j - 2]) : 0u;
+    wsel[c] = (uint16_t)(lo | ((lo | 8u) << 4) | ((4u + hi) << 8) | (((4u + hi) | 8u) << 12));
+  }
+  const uint32_t B = (uint32_t)a.bias;
+  const uint32_t BB = B * 0x00010001u, B3 = BB + 0x00030003u;
+  const uint32_t CU = (uint32_t)((4 * a.gap_open + 2) * 65537);
+  const uint32_t CL = (uint32_t)((4 * a.gap_open + 1) * 65537);
+  const uint32_t KU = (uint32_t)(4 * (a.gap_ext - a.gap_open));
+  const uint32_t KL = (uint32_t)(2 * (a.gap_ext - a.gap_open));
+  const uint32_t sm = (uint32_t)(uint8_t)(int8_t)(4 * a.match + 3);
+  const uint32_t sx = (uint32_t)(uint8_t)(int8_t)(4 * a.mismatch + 3);
+  const uint32_t all_x = sx * 0x01010101u;
+  const uint32_t SX = ((uint32_t)(4 * a.mismatch + 3) & 0xFFFFu) * 0x00010001u;
+  uint32_t pf0[RH], pf1[RH], h[RH], xl[RH];
+#pragma unroll
+  for (int k = 0; k < RH; ++k) {
+    const int i0 = 2 * tid * RH + k, i1 = i0 + RH;
+    pf0[k] = i0 < Q ? all_x ^ ((sm ^ sx) << (8 * class5((uint8_t)qg[i0]))) : all_x;
+    pf1[k] = i1 < Q ? all_x ^ ((sm ^ sx) << (8 * class5((uint8_t)qg[i1]))) : all_x;
+    h[k] = BB;
+    xl[k] = BB;
+  }
+  const int S4 = (R + 63 + 3) & ~3;
+  uint32_t* dirs = a.dirs + a.dir_off[item] + (int64_t)tid * S4;
+  __syncthreads();
+  const int act = min(kLW, (Q + 64 * RH - 1) / (64 * RH));  // warps with rows of the query
+  uint32_t send_u = BB, send_h = BB, diag = BB;
+  uint32_t bm = 0;         // maximum of the block's cells
+  uint32_t hs[3][RH];      // cells of the block's steps but the last
+  uint32_t W = B + 4;      // largest cell of the warp so far (from H = 1)
+  // the lane's maximum; its first row and column, or, while pending, the
+  // cells of the only 4 steps that hold it so far (snap, from step snap_s0)
+  uint32_t rv = 0;
+  int rr = 0, rc = 0, snap_s0 = 0;
+  bool pending = false;
+  uint32_t* snap = a.dirs + a.dir_off[item] + (int64_t)kLT * S4 + tid * (4 * RH);
+  // (rr, rc) takes the first cell of value rv in the 4 steps from s0 on
+  auto look_all = [&](int s0, const uint32_t* cells) {
+    for (int u = 0; u < 4; ++u)
+      for (int k = 0; k < RH; ++k) {
+        const uint32_t both = cells[u * RH + k];
+        for (int hf = 0; hf < 2; ++hf) {
+          const uint32_t c = hf ? both >> 16 : both & 0xFFFFu;
+          const int row = (2 * tid + hf) * RH + k + 1, col = s0 + u - 2 * lane + 1 - hf;
+          if (c == rv && row <= Q && col >= 1 && col <= R && (row < rr || (row == rr && col < rc))) {
+            rr = row;
+            rc = col;
+          }
+        }
+      }
+  };
+  auto step = [&](const int s, auto edge) -> uint32_t {
+    constexpr bool kEdge = decltype(edge)::value;
+    uint32_t ru = __shfl_up_sync(0xffffffffu, send_u, 1);
+    uint32_t rh = __shfl_up_sync(0xffffffffu, send_h, 1);
+    const int j = s - 2 * lane + 1;  // the low half's column; the high half's is j - 1
+    if (lane == 0) {
+      ru = rh = BB;  // row 0
+      if (warp > 0 && (!kEdge || j <= R)) {
+        const uint32_t x = ring[(warp - 1) * kRing16 + (j & (kRing16 - 1))];
+        ru = x << 16;
+        rh = x;
+      }
+    }
+    uint32_t up = __funnelshift_r(ru, send_u, 16);
+    const uint32_t hin = __funnelshift_r(rh, send_h, 16);
+    const uint32_t ws = wsel[kPad16 + j];
+    uint32_t in = 0;  // halves whose column lies inside the window
+    if (kEdge) in = (j >= 1 && j <= R ? 0xFFFFu : 0u) | (j >= 2 && j <= R + 1 ? 0xFFFF0000u : 0u);
+    uint32_t dg = diag, acc = 0, pair = 0;
+#pragma unroll
+    for (int k = 0; k < RH; ++k) {
+      uint32_t sc = prmt_b(pf0[k], pf1[k], ws);
+      if (kEdge) sc = (sc & in) | (SX & ~in);
+      const uint32_t dl = __viaddmax_s16x2(dg, sc, xl[k] + CL);
+      const uint32_t hx = __vimax3_s16x2(dl, up + CU, B3);
+      dg = h[k];
+      const uint32_t hh = hx & 0xFFFCFFFCu;
+      h[k] = hh;
+      const uint32_t bu = ~hx & 0x00010001u, bl = ~hx & 0x00020002u;  // 1 UP, 2 LEFT
+      up = bu * KU + hh;
+      xl[k] = bl * KL + hh;
+      // the strip's codes, last row lowest (multiply-adds: FMA pipe)
+      acc = k == 0 ? bu : acc * a.four + bu;
+      acc = bl * a.one + acc;
+      if (k & 1)
+        bm = __vimax3_s16x2(bm, pair, hh);
+      else
+        pair = hh;
+    }
+    send_u = up;
+    send_h = h[RH - 1];
+    diag = hin;
+    if (lane == 31 && warp + 1 < act)
+      ring[warp * kRing16 + ((j - 1) & (kRing16 - 1))] = (up >> 16) | (send_h & 0xFFFF0000u);
+    return acc;
+  };
+  auto keep = [&](int u) {
+#pragma unroll
+    for (int k = 0; k < RH; ++k) hs[u][k] = h[k];
+  };
+  const int steps = R + 63;
+  const int n_stages = kLag16 * (act - 1) + (steps + kStage16 - 1) / kStage16;
+  for (int stage = 0; stage < n_stages; ++stage) {
+    const int s_lo = (stage - kLag16 * warp) * kStage16;
+    if (warp < act && s_lo >= 0 && s_lo < steps) {
+#pragma unroll 1
+      for (int s0 = s_lo; s0 < s_lo + kStage16; s0 += 4) {
+        uint4 v;
+        bm = 0;
+        if (s0 >= 63 && s0 + 3 <= R - 1) {
+          v.x = step(s0, std::false_type());
+          keep(0);
+          v.y = step(s0 + 1, std::false_type());
+          keep(1);
+          v.z = step(s0 + 2, std::false_type());
+          keep(2);
+          v.w = step(s0 + 3, std::false_type());
+        } else {
+          v.x = step(s0, std::true_type());
+          keep(0);
+          v.y = step(s0 + 1, std::true_type());
+          keep(1);
+          v.z = step(s0 + 2, std::true_type());
+          keep(2);
+          v.w = step(s0 + 3, std::true_type());
+        }
+        if (s0 < S4) __stcg(reinterpret_cast<uint4*>(dirs + s0), v);
+        const uint32_t most = max(bm & 0xFFFFu, bm >> 16);
+        if (__any_sync(0xffffffffu, most >= W)) {
+          if (most >= W && most >= rv) {
+            if (most > rv) {
+              rv = most;
+              pending = true;
+            } else {  // the same maximum again: the first of them so far
+              if (pending) {
+                rr = rc = 0x7fffffff;
+                look_all(snap_s0, snap);
+                pending = false;
+              }
+            }
+            uint32_t cells[4 * RH];
+#pragma unroll
+            for (int k = 0; k < RH; ++k) {
+              cells[k] = hs[0][k];
+              cells[RH + k] = hs[1][k];
+              cells[2 * RH + k] = hs[2][k];
+              cells[3 * RH + k] = h[k];
+            }
+            uint4* to = reinterpret_cast<uint4*>(snap);
+#pragma unroll
+            for (int q = 0; q < RH; ++q)
+              to[q] = make_uint4(cells[4 * q], cells[4 * q + 1], cells[4 * q + 2], cells[4 * q + 3]);
+            if (pending)
+              snap_s0 = s0;
+            else
+              look_all(s0, snap);
+          }
+          // (rows past the query and columns past the window stay below the
+          // pair's maximum, so W never passes it)
+          W = max(W, __reduce_max_sync(0xffffffffu, most));
+        }
+      }
+    }
+    __syncthreads();
+  }
+  // first maximum in row-major order over the CTA
+  if (pending) {
+    rr = rc = 0x7fffffff;
+    look_all(snap_s0, snap);
+  }
+  if (rr == 0x7fffffff) rv = 0;  // (past the query or the window only)
+  __shared__ uint32_t red_v[kLW];
+  __shared__ int red_r[kLW], red_c[kLW];
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) {
+    const uint32_t ov = __shfl_xor_sync(0xffffffffu, rv, d);
+    const int orr = __shfl_xor_sync(0xffffffffu, rr, d);
+    const int oc = __shfl_xor_sync(0xffffffffu, rc, d);
+    if (ov > rv || (ov == rv && orr < rr)) {
+      rv = ov;
+      rr = orr;
+      rc = oc;
+    }
+  }
+  if (lane == 0) {
+    red_v[warp] = rv;
+    red_r[warp] = rr;
+    red_c[warp] = rc;
+  }
+  __syncthreads();
+  if (tid == 0) {
+    for (int w = 1; w < kLW; ++w) {
+      if (red_v[w] > rv || (red_v[w] == rv && red_r[w] < rr)) {
+        rv = red_v[w];
+        rr = red_r[w];
+        rc = red_c[w];
+      }
+    }
+    const int score = rv > B ? (int)((rv - B) >> 2) : 0;
+    a.best[p] = make_int2(score, score > 0 ? rr * (R + 1) + rc : 0);
+  }
+}
+
+// rows of a half for a query: 2, 4, 6 or 8
+__host__ __device__ inline int long16_rows(int Q) { return 2 * ((Q + 1023) / 1024); }
+
+// Pairs of all sizes in one launch (largest first), so that small ones fill
+// the SMs that large ones leave free.
+__global__ void __launch_bounds__(kLT, 2) sw_long16_kernel(LongArgs a) {
+  extern __shared__ __align__(16) uint8_t smem[];
+  const int64_t item = (int64_t)blockIdx.x;
+  if (item >= a.n) return;
+  const int32_t p = a.list[item];
+  const int Q = a.q_len[p], R = a.r_len[p];
+  switch (long16_rows(Q)) {
+    case 2: long16_pair<2>(a, item, p, Q, R, smem); break;
+    case 4: long16_pair<4>(a, item, p, Q, R, smem); break;
+    case 6: long16_pair<6>(a, item, p, Q, R, smem); break;
+    default: long16_pair<8>(a, item, p, Q, R, smem); break;
+  }
+}
+
+// Traceback walk over the long kernels' direction codes (the same rules as
 // sw_walk_kernel), one warp per pair.
 //
 // A walk is a chain of dependent reads.  The warp fetches a tile of 256
@@ -266,19 +542,21 @@ __global__ void __launch_bounds__(kLT, 2) sw_long_kernel(LongArgs a) {
 // bytes there); the moves then run from shared memory, every lane alike,
 // until one leaves the tile.  (One thread per pair read four words at a time,
 // and some walk of its warp waited for memory on almost every move: 4.2 ms
-// for queries of 3 to 4 kb, 0.95 ms now.)
+// for queries of 3 to 4 kb, 0.9 ms now.)
 constexpr int kTileWords = 256;
+constexpr int kTileSteps = 32;  // of a stream: 16 columns a diagonal crosses in it, 9
+                                // and more before them, about 5 past (gaps)
+constexpr int kTileStreams = kTileWords / kTileSteps;
 constexpr int kTileBytes = 256;  // of query and of window, before the cell
 constexpr int kWalkWarps = 4;
 
-template <int RPL>
-__global__ void __launch_bounds__(kWalkWarps * 32) sw_long_walk_kernel(LongArgs a) {
-  // words per stream: the columns a diagonal crosses in RPL rows, 9 before
-  // them and about 5 past (gaps)
-  constexpr int kWords = RPL <= 4 ? 16 : 32, kStreams = kTileWords / kWords;
+// P16: the directions are sw_long16_kernel's; else sw_long_kernel's with rpl
+// rows per thread.
+template <bool P16>
+__global__ void __launch_bounds__(kWalkWarps * 32) sw_long_walk_kernel(LongArgs a, int rpl_of) {
   __shared__ __align__(16) uint32_t tile_all[kWalkWarps][kTileWords];
   __shared__ char q_all[kWalkWarps][kTileBytes], w_all[kWalkWarps][kTileBytes];
-  __shared__ int lo_all[kWalkWarps][kStreams];
+  __shared__ int lo_all[kWalkWarps][kTileStreams];
   const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t item = (int64_t)blockIdx.x * kWalkWarps + wib;
   if (item >= a.n) return;  // (no block-wide synchronisation below)
@@ -287,59 +565,66 @@ __global__ void __launch_bounds__(kWalkWarps * 32) sw_long_walk_kernel(LongArgs 
   int* lo = lo_all[wib];  // per stream: its first step in the tile
   const int32_t p = a.list[item];
   const int R = a.r_len[p];
+  const int rpl = P16 ? 2 * long16_rows(a.q_len[p]) : rpl_of, half = rpl / 2;
   const char* qg = a.qry + a.q_off[p];
   const char* wg = a.ref + a.r_off[p];
-  const int S4 = (R + 31 + 3) & ~3;
+  const int S4 = (R + (P16 ? 63 : 31) + 3) & ~3;
   const uint32_t* dirs = a.dirs + a.dir_off[item];
   const int W = R + 1;
-  int t0 = -1, rows0 = 0, cols0 = 0;  // the tile's first thread; bytes before row / column
-  auto fetch = [&](int i, int jj) {  // the tile from cell (i, jj) on
-    t0 = (i - 1) / RPL;
-    rows0 = i;
-    cols0 = jj;
-    const int k0 = (i - 1) - t0 * RPL;
-    __syncwarp();
-#pragma unroll
-    for (int v = 0; v < kTileWords / 128; ++v) {
-      const int at = (v * 32 + lane) * 4, m = at / kWords, t = t0 - m;
-      // the column at which a diagonal enters thread t's rows, as its step
-      const int enter = jj - (m == 0 ? 0 : k0 + 1 + (m - 1) * RPL) + (t & 31) - 1;
-      const int first = max((enter + 8 - (kWords - 1)) & ~3, 0);
-      const int s = first + (at & (kWords - 1));
-      uint4 x = make_uint4(0, 0, 0, 0);
-      if (t >= 0 && s + 4 <= S4)
-        x = __ldcg(reinterpret_cast<const uint4*>(dirs + (int64_t)t * S4 + s));
-      *reinterpret_cast<uint4*>(tile + at) = x;
-      if ((at & (kWords - 1)) == 0) lo[m] = first;
-    }
-    for (int b = lane; b < kTileBytes; b += 32) {
-      if (b < i) qs[b] = qg[i - 1 - b];
-      if (b < jj) ws[b] = wg[jj - 1 - b];
-    }
-    __syncwarp();
-  };
-  // the code of cell (i, jj); fetches a tile when it is not in this one
-  auto code_at = [&](int i, int jj) -> uint32_t {
-    const int t = (i - 1) / RPL, k = (i - 1) - t * RPL, step = jj + (t & 31) - 1;
-    int m = t0 - t;
-    if (t0 < 0 || m >= kStreams || step < lo[m] || step >= lo[m] + kWords ||
-        rows0 - i >= kTileBytes - 1 || cols0 - jj >= kTileBytes - 1) {
-      fetch(i, jj);
-      m = 0;
-    }
-    return (tile[m * kWords + (step - lo[m])] >> (2 * k)) & 3u;
-  };
-  enum : int { kNone = 0, kDiag = 1, kUp = 2, kLeft = 3 };
-  auto dir_of = [](uint32_t code, int h) -> int {
-    return code == 2u ? kDiag : code == 1u ? kUp : (h == 0 ? kNone : kLeft);
-  };
-  const int m = a.match, x = a.mismatch, o = a.gap_open, e = a.gap_ext;
-  char* qc = a.qcons ? a.qcons + (int64_t)p * a.cons_stride : nullptr;
-  char* rc = a.rcons ? a.rcons + (int64_t)p * a.cons_stride : nullptr;
   const int2 b = a.best[p];
   int cr = b.y / W, cc = b.y % W;
   int h = b.x;
-  int d = (cr == 0 || cc == 0) ? kNone : dir_of(code_at(cr, cc), h);
+  // the cell's thread, row in it, and wavefront lane
+  int t = cr > 0 ? (cr - 1) / rpl : 0, k = cr > 0 ? (cr - 1) - t * rpl : 0;
+  auto lane_of = [&](int tt, int kk) -> int {
+    return P16 ? 2 * (tt & 31) + (kk >= half ? 1 : 0) : tt & 31;
+  };
+  int wl = lane_of(t, k);
+  int m = kTileStreams, lo_m = 0;  // its stream in the tile (none yet) and that one's first step
+  int rows0 = 0, cols0 = 0;        // the tile's cell
+  auto fetch = [&]() {  // the tile from the cell on
+    rows0 = cr;
+    cols0 = cc;
+    __syncwarp();
+#pragma unroll
+    for (int v = 0; v < kTileWords / 128; ++v) {
+      const int at = (v * 32 + lane) * 4, st = at / kTileSteps, tt = t - st;
+      // the step at which a diagonal enters thread tt's rows
+      const int enter = st == 0 ? cc + wl - 1 : cc - (k + 1 + (st - 1) * rpl) + lane_of(tt, rpl - 1) - 1;
+      const int first = max((enter + 8 - (kTileSteps - 1)) & ~3, 0);
+      const int s = first + (at & (kTileSteps - 1));
+      uint4 x = make_uint4(0, 0, 0, 0);
+      if (tt >= 0 && s + 4 <= S4)
+        x = __ldcg(reinterpret_cast<const uint4*>(dirs + (int64_t)tt * S4 + s));
+      *reinterpret_cast<uint4*>(tile + at) = x;
+      if ((at & (kTileSteps - 1)) == 0) lo[st] = first;
+    }
+    for (int i = lane; i < kTileBytes; i += 32) {
+      if (i < cr) qs[i] = qg[cr - 1 - i];
+      if (i < cc) ws[i] = wg[cc - 1 - i];
+    }
+    __syncwarp();
+    m = 0;
+    lo_m = lo[0];
+  };
+  // the cell's code (a tile holds at most 128 rows and 160 columns, so its
+  // bytes too)
+  auto code = [&]() -> uint32_t {
+    if (m >= kTileStreams || (uint32_t)(cc + wl - 1 - lo_m) >= (uint32_t)kTileSteps) fetch();
+    const uint32_t word = tile[m * kTileSteps + (cc + wl - 1 - lo_m)];
+    const int sh = !P16 ? 2 * k : k >= half ? 16 + 2 * (rpl - 1 - k) : 2 * (half - 1 - k);
+    return (word >> sh) & 3u;
+  };
+  enum : int { kNone = 0, kDiag = 1, kUp = 2, kLeft = 3 };
+  constexpr uint32_t kUpCode = 1u, kLeftCode = P16 ? 2u : 0u;
+  auto dir_of = [](uint32_t c, int hh) -> int {
+    if (P16) return c == kUpCode ? kUp : c == kLeftCode ? kLeft : (hh == 0 ? kNone : kDiag);
+    return c == 2u ? kDiag : c == kUpCode ? kUp : (hh == 0 ? kNone : kLeft);
+  };
+  const int ma = a.match, x = a.mismatch, o = a.gap_open, e = a.gap_ext;
+  char* qc = a.qcons ? a.qcons + (int64_t)p * a.cons_stride : nullptr;
+  char* rc = a.rcons ? a.rcons + (int64_t)p * a.cons_stride : nullptr;
+  int d = (cr == 0 || cc == 0) ? kNone : dir_of(code(), h);
   int tick = -1, nref = -1, start = 0;
   char my_q = 0, my_r = 0;  // the bytes of move tick with tick % 32 == lane
   while (d != kNone) {
@@ -359,13 +644,23 @@ __global__ void __launch_bounds__(kWalkWarps * 32) sw_long_walk_kernel(LongArgs 
     cr -= up ? 1 : 0;
     cc -= left ? 1 : 0;
     if (cr == 0 || cc == 0) break;
-    const uint32_t pc = code_at(cr, cc);
+    if (up) {
+      if (--k < 0) {
+        k = rpl - 1;
+        --t;
+        wl = lane_of(t, k);
+        if (++m < kTileStreams) lo_m = lo[m];
+      } else if (P16 && k == half - 1) {
+        --wl;
+      }
+    }
+    const uint32_t pc = code();
     if (d == kDiag) {
       const int uq = upcase((uint8_t)qb), ur = upcase((uint8_t)rb);
-      h -= (uq == ur || uq == 'N' || ur == 'N') ? m : x;
+      h -= (uq == ur || uq == 'N' || ur == 'N') ? ma : x;
     } else {
       // the gap costs gap_ext when the predecessor itself moved the same way
-      h -= (d == kUp ? pc == 1u : pc == 0u) ? e : o;
+      h -= (d == kUp ? pc == kUpCode : pc == kLeftCode) ? e : o;
     }
     d = dir_of(pc, h);
   }
@@ -390,9 +685,7 @@ int launch_long_rpl(cudaStream_t st, const LongArgs& a, bool prof) {
     sw_long_kernel<RPL, true><<<(unsigned)a.n, kLT, smem, st>>>(a);
   else
     sw_long_kernel<RPL, false><<<(unsigned)a.n, kLT, smem, st>>>(a);
-  sw_long_walk_kernel<RPL><<<(unsigned)((a.n + kWalkWarps - 1) / kWalkWarps), kWalkWarps * 32, 0,
-                             st>>>(a);
-  return 2;
+  return 1;
 }
 
 }  // namespace
@@ -401,7 +694,8 @@ int long_rows_per_lane(int Q) {
   return Q <= 4 * kLT ? 4 : Q <= 8 * kLT ? 8 : Q <= 12 * kLT ? 12 : Q <= 16 * kLT ? 16 : 0;
 }
 
-int64_t long_slot_words(int R) { return (int64_t)kLT * ((R + 31 + 3) & ~3); }
+// (and 32 words a thread for the cells sw_long16_kernel puts aside)
+int64_t long_slot_words(int R) { return (int64_t)kLT * (((R + 63 + 3) & ~3) + 32); }
 
 int long_bias(int gap_open) { return ((-(16 * gap_open + 1)) + 15) & ~15; }
 
@@ -410,20 +704,42 @@ bool long_prof_ok(int m, int x, int gap_open, int max_q) {
          16ll * m * max_q + long_bias(gap_open) + 16 < (1ll << 18);
 }
 
-int launch_sw_long(cudaStream_t st, const LongArgs& a, int rpl, bool prof) {
-  if (a.n <= 0) return 0;
+static int long16_bias(int gap_open) { return ((-(4 * gap_open + 1)) + 3) & ~3; }
+
+int long16_max_q(int m, int x, int o, int e) {
+  if (!(m > 0 && x < 0 && o < 0 && e < 0 && e >= o)) return 0;
+  if (4 * m + 3 > 127 || 4 * x + 3 < -128 || o < -4096) return 0;
+  // the largest cell, 4 m Q + B + 3, and its gap candidates stay below 2^15
+  const int room = 32767 - long16_bias(o) - 4 * (e - o) - 8;
+  return room <= 0 ? 0 : room / (4 * m);
+}
+
+int launch_sw_long(cudaStream_t st, const LongArgs& args, int rpl, int kind) {
+  if (args.n <= 0) return 0;
   // shared memory: window (2 B per column) + rings, 23 KB at the longest window
-  if (((2 * (a.max_r + 1) + 15) & ~15) + (kLW - 1) * 2 * kRing * 4 > 48 * 1024) return 0;
-  if (prof && (a.bias != long_bias(a.gap_open) ||
-               !long_prof_ok(a.match, a.mismatch, a.gap_open, 256 * rpl)))
-    return 0;
-  switch (rpl) {
-    case 4: return launch_long_rpl<4>(st, a, prof);
-    case 8: return launch_long_rpl<8>(st, a, prof);
-    case 12: return launch_long_rpl<12>(st, a, prof);
-    case 16: return launch_long_rpl<16>(st, a, prof);
-    default: return 0;
+  if (((2 * (args.max_r + kSel16) + 15) & ~15) + (kLW - 1) * 2 * kRing * 4 > 48 * 1024) return 0;
+  LongArgs a = args;
+  a.one = 1;
+  a.four = 4;
+  a.bias = kind == kLong16 ? long16_bias(a.gap_open) : long_bias(a.gap_open);
+  if (kind == kLongProf && !long_prof_ok(a.match, a.mismatch, a.gap_open, 256 * rpl)) return 0;
+  if (kind == kLong16 && long16_max_q(a.match, a.mismatch, a.gap_open, a.gap_ext) <= 0) return 0;
+  const unsigned walks = (unsigned)((a.n + kWalkWarps - 1) / kWalkWarps);
+  if (kind == kLong16) {
+    const size_t smem = ((2 * (a.max_r + kSel16) + 15) & ~15) + (size_t)(kLW - 1) * kRing16 * 4;
+    sw_long16_kernel<<<(unsigned)a.n, kLT, smem, st>>>(a);
+    sw_long_walk_kernel<true><<<walks, kWalkWarps * 32, 0, st>>>(a, 0);
+    return 2;
   }
+  const bool prof = kind == kLongProf;
+  const int k = rpl == 4    ? launch_long_rpl<4>(st, a, prof)
+                : rpl == 8  ? launch_long_rpl<8>(st, a, prof)
+                : rpl == 12 ? launch_long_rpl<12>(st, a, prof)
+                : rpl == 16 ? launch_long_rpl<16>(st, a, prof)
+                            : 0;
+  if (k == 0) return 0;
+  sw_long_walk_kernel<false><<<walks, kWalkWarps * 32, 0, st>>>(a, rpl);
+  return 2;
 }
 
 }  // namespace swift

@@ -2337,6 +2337,10 @@ static int align_resident_impl(swift_ctx* ctx, const swift_index* idx, const swi
     for (const WaveReq& q : *wave) min_q = std::min(min_q, (int)q.Q);
   const bool gapless = fast_ok && ctx->sw_path == 0 && max_mis >= 0 && idx->d_odd && nproc > 0 &&
                        min_q <= kWin - kShiftBases + max_mis;
+  // ... and the diagonals of such reads are left to the LCS bound (251-base
+  // reads 5.9 -> 4.4 ms; after a first pass that took them it settles too few
+  // more: 1 M x 100 bases 46 us less of trace for 231 us)
+  const bool cut_reads = Q > kWin - kShiftBases + max_mis;
   FormatArgs all;
   memset(&all, 0, sizeof(all));
   all.reads = rd->d_bytes;
@@ -2492,7 +2496,8 @@ static int align_resident_impl(swift_ctx* ctx, const swift_index* idx, const swi
   // generic kernel (full result at once)
   // counters: 0 packed-path pairs, 1 generic pairs, 2 trace list,
   // 3 pairs the LCS bound keeps (exact-score list), 4 second trace list,
-  // 5 printed records
+  // 5 printed records, 6 pairs of list 2 (SAM: 0) that the gapless
+  // pass by the LCS bound leaves
   // counters 8.. : histogram and fill of the early-stop sort (two uses)
   int32_t *fast_list, *gen_list, *tb_list, *cnt;
   CK(sc.get(&fast_list, nn));
@@ -2684,7 +2689,8 @@ static int align_resident_impl(swift_ctx* ctx, const swift_index* idx, const swi
     if (fast_ok && n > 0) {
       CK(rb.get(h_cnt, cnt, sizeof(h_cnt)));
       CK(rb.sync());
-      int32_t* sam_list = fast_list;
+      int32_t *sam_list = fast_list, *sam_count = cnt;
+      int64_t sam_traced = h_cnt[0];
       if (lsuf) {
         // suffix LCS values for the early stop, then the order that groups
         // pairs stopping alike
@@ -2695,12 +2701,28 @@ static int align_resident_impl(swift_ctx* ctx, const swift_index* idx, const swi
         if (k == 0) return fail(ctx, SWIFT_E_DEVICE, "LCS pass could not launch");
         launches += k;
         CKLAUNCH();
-        rc = sort_by_stop(fast_list, cnt, h_cnt[0], sorted, true);
+        // (reads cut off by their windows: as the candidates below)
+        int64_t sam_n = h_cnt[0];
+        int32_t *from = fast_list, *from_n = cnt;
+        if (cut_reads) {
+          if (launch_gapless_bound(st, fa2, sam_n, tb_list, cnt + 6) == 0)
+            return fail(ctx, SWIFT_E_DEVICE, "gapless pass could not launch");
+          CKLAUNCH();
+          ++launches;
+          CK(rb.get(h_cnt, cnt, sizeof(h_cnt)));
+          CK(rb.sync());
+          sam_n = h_cnt[6];
+          from = tb_list;
+          from_n = cnt + 6;
+        }
+        rc = sort_by_stop(from, from_n, sam_n, sorted, true);
         if (rc != SWIFT_OK) return rc;
         sam_list = sorted;
+        sam_count = from_n;
+        sam_traced = sam_n;
       }
       fa2.cells_done = d_cells + 1;
-      rc = trace_list(sam_list, cnt, h_cnt[0], true);
+      rc = trace_list(sam_list, sam_count, sam_traced, true);
       if (rc != SWIFT_OK) return rc;
       fa2.cells_done = d_cells;
       fa2.lsuf = nullptr;
@@ -2719,18 +2741,30 @@ static int align_resident_impl(swift_ctx* ctx, const swift_index* idx, const swi
     launch_candidates(st, fa, tb_list, cnt + 2);
     CKLAUNCH();
     ++launches;
+    int32_t *cand_list = tb_list, *cand_count = cnt + 2;
+    if (cut_reads) {
+      // their own diagonals settle most of such reads' candidates
+      fa2.list = tb_list;
+      fa2.count = cnt + 2;
+      fa2.list_offset = 0;
+      cand_list = gen_list;  // free: the generic kernel has run
+      cand_count = cnt + 6;
+      if (launch_gapless_bound(st, fa2, n, cand_list, cand_count) == 0)
+        return fail(ctx, SWIFT_E_DEVICE, "gapless pass could not launch");
+      CKLAUNCH();
+      ++launches;
+    }
     CK(rb.get(h_cnt, cnt, sizeof(h_cnt)));
     CK(rb.sync());
     CK(cudaEventRecord(ctx->ev[6], st));
-    cand_n = h_cnt[2];
+    cand_n = cut_reads ? h_cnt[6] : h_cnt[2];
     fa2.cells_done = d_cells + 1;
-    int32_t* cand_list = tb_list;
     if (lsuf) {
-      rc = sort_by_stop(tb_list, cnt + 2, cand_n, sorted, true);
+      rc = sort_by_stop(cand_list, cand_count, cand_n, sorted, true);
       if (rc != SWIFT_OK) return rc;
       cand_list = sorted;
     }
-    rc = trace_list(cand_list, cnt + 2, cand_n, true);
+    rc = trace_list(cand_list, cand_count, cand_n, true);
     if (rc != SWIFT_OK) return rc;
     fa2.cells_done = d_cells;
     // pairs whose LCS bound cannot rule them out against their candidate's

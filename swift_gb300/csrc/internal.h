@@ -649,6 +649,10 @@ int launch_sw_trace(cudaStream_t st, const FastArgs& a, int64_t max_pairs,
 // sw_lcs.cu: a.ub[p] = match * LCS(query, window) for the listed pairs, and
 // with a.lsuf the suffix LCS values
 int launch_sw_lcs(cudaStream_t st, const FastArgs& a, int64_t max_pairs);
+// ungapped.cu: after the LCS pass (a.ub), the listed pairs whose alignment
+// holds no gap (result and strings written) and, in rest, the others
+int launch_gapless_bound(cudaStream_t st, const FastArgs& a, int64_t max_pairs, int32_t* rest,
+                         int32_t* n_rest);
 int measure_dpx_peak(cudaStream_t st, int device, double* lane_instr_per_s);
 
 // out.cu

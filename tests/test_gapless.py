@@ -13,6 +13,7 @@ lower case and N nearby, scorings at and past its mismatch limit.
 """
 import random
 
+import numpy as np
 import pytest
 
 
@@ -207,3 +208,25 @@ def test_paired_steps(ctx, sg, oracle, L, frag):
         got = ctx.align_paired(ix, r1, r2, sg.default_params(out_format=fmt), *frag)
         o = oracle.default_params(device_mem=ctx.info()["total_mem"], out_format=fmt)
         assert got == oracle.align_paired(ref, r1, r2, o, *frag)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("L,sub", [(60, 0.05), (100, 0.04), (201, 0.01), (230, 0.02), (251, 0.01),
+                                   (300, 0.03)])
+def test_settled_by_the_lcs_bound(ctx, sg, L, sub):
+    # reads the first pass leaves (more mismatches than it takes, or cut off
+    # by their window) in numbers that run the LCS pass: as the int32 kernel
+    from swift_gb300 import synth
+    names, seqs = synth.make_reference(200_000, 3, sigma=0.4, repeat_frac=0.2, n_units=15, seed=L)
+    seqs[0][5000:5900] = np.frombuffer(b"ACGTTGCAAC" * 90, np.uint8)  # diagonals alike
+    rn, rs, _ = synth.make_reads(seqs, 9000, L, sub, 0.0005, 0.05, seed=L + 1)
+    reads = synth.reads_fasta(rn, rs)
+    ix = ctx.index(synth.fasta_bytes(names, seqs))
+    for kw in (dict(), dict(out_format=1), dict(match=3, mismatch=-2, gap_open=-6, gap_ext=-2)):
+        p = sg.default_params(max_read_len=300, **kw)
+        got = ctx.align(ix, reads, p)
+        ctx.set_sw_path(1)
+        try:
+            assert got == ctx.align(ix, reads, p), kw
+        finally:
+            ctx.set_sw_path(0)

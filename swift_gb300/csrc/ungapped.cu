@@ -26,13 +26,14 @@
 // 16..31 of the query are compared with the window at every start by a
 // funnel shift, an exclusive or and a population count (8 instructions per
 // diagonal), and a diagonal with at most k mismatches there (one in 30,000
-// by chance) is checked whole.
+// by chance) is checked whole, after the scan.
 //
 // Layout: one thread per record; the codes of the reference (16 bases a
 // word, in L2) and of the reads, both strands, are read in place, so no
 // window or query is written out for the records this settles.  Bound by
-// issue: at 100-base reads and 300-base windows about 2,000 instructions a
-// record, against 190,000 for the trace pass's share of a pair.
+// the ALU pipe (84 %): at 100-base reads and 300-base windows about 2,000
+// instructions a record, against 190,000 for the trace pass's share of a pair
+// (4.13 M records 0.56 ms).
 //
 // gapless_bound_kernel applies the same argument with a smaller bound to the
 // pairs that remain, once the LCS pass has run: the matches of a chain are a
@@ -221,7 +222,11 @@ __global__ void __launch_bounds__(kGaplessThreads) gapless_kernel(GaplessArgs a)
       }
       run_to(Q);
     };
-    // rows 16..31 against the window at columns p = 16 + d
+    // rows 16..31 against the window at columns p = 16 + d; the diagonals
+    // that pass are checked after the scan, all lanes of the warp together
+    // (at once, each alone, they took two thirds of the kernel)
+    uint64_t found = 0;
+    int n_found = 0;
     const uint32_t qa = q[1];
     const int p_lo = 16 - k, p_hi = 16 + R - Q + k;
     uint32_t lo = raw(0), hi = raw(1);
@@ -237,9 +242,16 @@ __global__ void __launch_bounds__(kGaplessThreads) gapless_kernel(GaplessArgs a)
       w0 = w1;
       for (; hits; hits &= hits - 1) {
         const int p = 16 * t + __ffs(hits) - 1;
-        if (p >= p_lo && p <= p_hi) check(p - 16);
+        if (p < p_lo || p > p_hi) continue;
+        if (n_found < 4) {
+          found |= (uint64_t)p << (16 * n_found);
+          ++n_found;
+        } else {
+          check(p - 16);
+        }
       }
     }
+    for (int f = 0; f < n_found; ++f) check((int)((found >> (16 * f)) & 0xFFFFu) - 16);
     if (best_row > 0) {
       state = kGaplessDone;
       al.score = best;

@@ -2551,7 +2551,9 @@ static int align_resident_impl(swift_ctx* ctx, const swift_index* idx, const swi
   // suffix LCS values: early stop of the score and trace passes (bounded
   // selection; every pair traced with SAM output)
   uint16_t* lsuf = nullptr;
-  const bool lcs_stop = fast_ok && ctx->sw_path == 0 && !direct;
+  // (not with SAM output behind the gapless pass: what that leaves seldom
+  // stops early, and the tests cost more than they save)
+  const bool lcs_stop = fast_ok && ctx->sw_path == 0 && !direct && !(sam && !cut_reads);
   if (bounded) CK(sc.get(&cand, nn));
   if (lcs_stop) {
     CK(sc.get(&ub, nn));

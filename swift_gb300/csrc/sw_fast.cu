@@ -56,7 +56,8 @@ Shape shape_of(const FastArgs& a) {
 template <bool TRACE, bool VAR>
 int launch_shape(cudaStream_t st, const FastArgs& a, int64_t max_pairs) {
   const Shape s = shape_of(a);
-  if (s.G == 0 || max_pairs <= 0) return 0;
+  if (s.G == 0 || max_pairs <= 0 || a.R > kFastMaxR) return 0;
+  if (((a.w_stride | (int64_t)(uintptr_t)a.w) & 15) != 0) return 0;  // 16-byte loads of the windows
   const int pairs_per_warp = 2 * (32 / s.G);
   const int64_t warps = (max_pairs + pairs_per_warp - 1) / pairs_per_warp;
   const unsigned grid = (unsigned)((warps + kPkWarps - 1) / kPkWarps);
@@ -184,8 +185,11 @@ int packed_shape_candidates(int Q, int32_t* g, int32_t* rpl, int cap) {
 }
 
 int launch_sw_score(cudaStream_t st, const FastArgs& a, int64_t max_pairs) {
-  return a.q_len ? launch_shape<false, true>(st, a, max_pairs)
-                 : launch_shape<false, false>(st, a, max_pairs);
+  FastArgs b = a;
+  b.one = 1;
+  b.four = 4;
+  return a.q_len ? launch_shape<false, true>(st, b, max_pairs)
+                 : launch_shape<false, false>(st, b, max_pairs);
 }
 
 int launch_sw_trace(cudaStream_t st, const FastArgs& a, int64_t max_pairs, cudaEvent_t before,

@@ -64,6 +64,9 @@ __device__ __forceinline__ uint32_t base_class(uint32_t c) {
   return u == 'C' ? 1u : u == 'G' ? 2u : u == 'T' ? 3u : 0u;
 }
 
+// base_class of four ACGTacgt bytes
+__device__ __forceinline__ uint32_t base_class4(uint32_t x) { return ((x >> 1) ^ (x >> 2)) & 0x03030303u; }
+
 // per-half 0xFFFF where a > b, for non-negative 16-bit integers below 0x7C00
 __device__ __forceinline__ uint32_t gt_mask(uint32_t a, uint32_t b) {
   uint32_t d;
@@ -140,10 +143,34 @@ __device__ __forceinline__ void packed_item(const FastArgs& a, const int64_t war
   const char* w0 = a.w + (int64_t)p0 * a.w_stride;
   const char* w1 = a.w + (int64_t)p1 * a.w_stride;
   uint32_t* wsel = wsel_all + (wib * kGroups + g) * (a.R + 1);
-  for (int c = sl; c < R; c += G) {
-    uint32_t s0 = (!VAR || c < R0) ? base_class((uint8_t)w0[c]) : 0u;
-    uint32_t s1 = (!VAR || c < R1) ? base_class((uint8_t)w1[c]) : 0u;
-    wsel[c + 1] = s0 | ((s0 | 8u) << 4) | ((4u + s1) << 8) | (((4u + s1) | 8u) << 12);
+  // Selectors of the two windows, 16 columns per lane and round: every load
+  // goes out before the first is used (rows are 16-byte aligned; byte by byte
+  // a warp waited for memory 11 % of its time).  Columns past a pair's own
+  // window hold any base; they are never used.
+  {
+    constexpr int kRounds = (kFastMaxR / 16 + G - 1) / G;
+    uint4 x0[kRounds], x1[kRounds];
+#pragma unroll
+    for (int r = 0; r < kRounds; ++r) {
+      const int c = 16 * (sl + G * r);
+      x0[r] = c < R0 ? __ldg(reinterpret_cast<const uint4*>(w0 + c)) : make_uint4(0, 0, 0, 0);
+      x1[r] = c < R1 ? __ldg(reinterpret_cast<const uint4*>(w1 + c)) : make_uint4(0, 0, 0, 0);
+    }
+#pragma unroll
+    for (int r = 0; r < kRounds; ++r) {
+      const int c = 16 * (sl + G * r);
+      const uint32_t y0[4] = {x0[r].x, x0[r].y, x0[r].z, x0[r].w};
+      const uint32_t y1[4] = {x1[r].x, x1[r].y, x1[r].z, x1[r].w};
+      if (c < R) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          const uint32_t s0 = (base_class4(y0[i >> 2]) >> (8 * (i & 3))) & 3u;
+          const uint32_t s1 = (base_class4(y1[i >> 2]) >> (8 * (i & 3))) & 3u;
+          // nibbles s0, s0 | 8, 4 + s1, (4 + s1) | 8
+          if (c + i < R) wsel[c + i + 1] = s0 * 0x11u + s1 * 0x1100u + 0xC480u;
+        }
+      }
+    }
   }
   __syncwarp();
   const uint32_t B = (uint32_t)a.bias;

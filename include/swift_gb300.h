@@ -232,7 +232,7 @@ int swift_sw_batch_noalloc(swift_ctx *ctx, const char *qry, const char *ref, int
 typedef struct {
   double ms;               /* device time of the call (CUDA events)           */
   int64_t pairs, cells;    /* cells = sum over pairs of q_len * r_len         */
-  int64_t segments;        /* groups of one shape, one launch set each        */
+  int64_t segments;        /* groups of pairs, one launch set each            */
   int64_t generic_pairs;   /* pairs on the int32 kernel                       */
   int64_t launches;        /* kernels this library launched                   */
   /* the packed shape (lanes, rows per lane) each query class ran with
@@ -244,12 +244,13 @@ typedef struct {
 } swift_pairs_stats;
 
 /* Packed-shape choice of swift_sw_pairs: 1 (default) times the candidate
- * (lanes, rows per lane) shapes of each row class and window bin (with at
- * least 1,024 pairs) on a sample of the call's pairs the first time the
- * context meets them, and
- * keeps the fastest for the context; 0 uses the fixed default shapes;
- * k >= 2 runs the (k - 2)-th candidate of every class (the default when it
- * has fewer).  All give identical results. */
+ * (lanes, rows per lane) shapes of each launch's rows and window bin on a
+ * sample of the call's pairs the first time the context meets them, and
+ * keeps the fastest for the context; row classes of few pairs share a launch,
+ * and launches of under 2,048 pairs take a shape for few pairs untimed.
+ * 0 uses the fixed default shape of every row class; k >= 2 runs the
+ * (k - 2)-th candidate of every class (the default when it has fewer).  All
+ * give identical results. */
 int swift_ctx_set_tuning(swift_ctx *ctx, int32_t mode);
 
 /* Phase 2 on explicit pairs of varying lengths: the batched form of

@@ -415,6 +415,11 @@ constexpr int64_t kFewGeneric = 1024;
 // packed; 4,096: 92 each; 2,048 of 100 x 300: 143 each; 2,048 of 250 x 500:
 // 511 against 306; 1,024 of 250 x 500: 271 against 290).
 constexpr int64_t kBatchPackedPairs = 2048, kBatchPackedRows = 200000;
+// swift_sw_pairs: its launches alternate between two streams from here on
+constexpr int64_t kAlternatePairs = 1024;
+// and classes of fewer pairs than kMergePairs share a launch; launches of
+// fewer than kTunePairs take the shape for few pairs, others are tuned
+constexpr int64_t kMergePairs = 4096, kTunePairs = 2048;
 
 struct SeedOut {
   int32_t *m_read = nullptr, *m_strand = nullptr, *m_ri = nullptr, *m_sh = nullptr,
@@ -1890,7 +1895,13 @@ int swift_sw_pairs(swift_ctx* ctx, const char* qry, const int64_t* q_off, const 
         }
         const bool gen = (hk[s] >> 20) & 1;
         const int q = (hk[s] >> 11) & 511, R = hk[s] & 2047;
-        if (!gen && !groups.empty() && !groups.back().gen && groups.back().Q == 8 * q) {
+        // a class of few pairs goes on with the next one (in the taller
+        // shape, by per-pair lengths): launches of a few thousand pairs last
+        // as long as one pair does, 20 classes of them 2.4 ms
+        const bool few = ctx->tuning == 1 && !groups.empty() && groups.back().count < kMergePairs &&
+                         (groups.back().Q <= 128) == (8 * q <= 128);
+        if (!gen && !groups.empty() && !groups.back().gen && (groups.back().Q == 8 * q || few)) {
+          groups.back().Q = 8 * q;
           groups.back().R = std::max(groups.back().R, R);
           groups.back().count += hc[s];
           continue;
@@ -1904,90 +1915,73 @@ int swift_sw_pairs(swift_ctx* ctx, const char* qry, const int64_t* q_off, const 
       int32_t* gcount_d = seg_count;  // reuse: the segment counts are on the host now
       if (!groups.empty())
         CK(cudaMemcpyAsync(gcount_d, gcount.data(), groups.size() * 4, cudaMemcpyHostToDevice, st));
+      // packed trace pass + walk over pairs of one class, per-pair lengths,
+      // in sub-chunks that bound the direction scratch
+      const int64_t sub = 262144;
+      // a class's (lanes, rows per lane) shape: the default (0, 0), a forced
+      // candidate, or the fastest candidate on a sample of these pairs
+      // (timed once per context, class and window bin)
+      struct Plan {
+        int bias = 0, g = 0, rpl = 0;
+        bool tune = false;
+      };
+      std::vector<Plan> plans(groups.size());
+      int64_t words = 0, packed_launches = 0, packed_pairs = 0;
       for (size_t gi = 0; gi < groups.size(); ++gi) {
         const Group& G = groups[gi];
-        const int Q = G.Q, R = G.R;
-        const int64_t cnt = G.count;
-        int32_t* list = sorted + G.start;
-        int bias = 0;
-        if (G.gen || !fast_params_ok(Q, R, m, x, o, e, &bias)) {
-          // (a packed class whose longest query the packed scoring does not
-          // take runs here too: the int32 kernel takes per-launch shapes, so
-          // its pairs go one exact shape at a time)
-          if (!G.gen) return fail(ctx, SWIFT_E_DEVICE, "packed class outside the packed scoring");
-          SwArgs sa;
-          memset(&sa, 0, sizeof(sa));
-          sa.q = qbuf;
-          sa.w = wbuf;
-          sa.q_stride = q_stride;
-          sa.w_stride = w_stride;
-          sa.Q = Q;
-          sa.R = R;
-          sa.match = m;
-          sa.mismatch = x;
-          sa.gap_open = o;
-          sa.gap_ext = e;
-          sa.n = cnt;
-          sa.aln = aln;
-          sa.qcons = cq;
-          sa.rcons = cr;
-          sa.cons_stride = cs;
-          sa.list = list;
-          sa.count = gcount_d + gi;
-          int rc = launch_sw(st, sa, &ctx->err);
-          if (rc != SWIFT_OK) return rc;
-          CKLAUNCH();
-          ++launches;
-          ps.generic_pairs += cnt;
-          continue;
-        }
-        // packed trace pass + walk over pairs of one class, per-pair lengths,
-        // in sub-chunks that bound the direction scratch
-        const int64_t sub = 262144;
-        // the class's (lanes, rows per lane) shape: the default, a forced
-        // candidate, or the fastest candidate on a sample of these pairs
-        // (timed once per context, class and window bin)
+        Plan& pl = plans[gi];
+        if (G.gen) continue;
+        // (a packed class whose longest query the packed scoring does not
+        // take runs on the int32 kernel, its pairs keyed one exact shape at
+        // a time)
+        if (!fast_params_ok(G.Q, G.R, m, x, o, e, &pl.bias))
+          return fail(ctx, SWIFT_E_DEVICE, "packed class outside the packed scoring");
         int32_t cg[16], crpl[16];
-        const int ncand = packed_shape_candidates(Q, cg, crpl, 16);
-        int sg = 0, srpl = 0;
+        const int ncand = packed_shape_candidates(G.Q, cg, crpl, 16);
         if (ctx->tuning >= 2 && ctx->tuning - 2 < ncand) {
-          sg = cg[ctx->tuning - 2];
-          srpl = crpl[ctx->tuning - 2];
+          pl.g = cg[ctx->tuning - 2];
+          pl.rpl = crpl[ctx->tuning - 2];
         }
-        const int tkey = (Q / 8) * 64 + (R + 63) / 64;
-        const bool tune = ctx->tuning == 1 && ncand > 1 && !ctx->tuned.count(tkey) &&
-                          cnt >= 1024;
-        if (ctx->tuning == 1 && !tune) {
-          auto it = ctx->tuned.find(tkey);
+        if (ctx->tuning == 1 && G.count < kTunePairs) {
+          few_pairs_shape(G.Q, G.count, &pl.g, &pl.rpl);
+        } else if (ctx->tuning == 1) {
+          auto it = ctx->tuned.find((G.Q / 8) * 64 + (G.R + 63) / 64);
           if (it != ctx->tuned.end()) {
-            sg = it->second.first;
-            srpl = it->second.second;
+            pl.g = it->second.first;
+            pl.rpl = it->second.second;
+          } else {
+            pl.tune = ncand > 1;
           }
         }
         // scratch for the shape that will run, or every one the tuner tries
-        int64_t words = 0;
-        for (int c = 0; c < (tune ? ncand : 1); ++c)
-          words = std::max(words, trace_scratch_words(Q, R, std::min(cnt, sub),
-                                                      tune ? cg[c] : sg, tune ? crpl[c] : srpl));
-        if (words > dirs_words[0]) {
-          CK(sc.get(&dirs[0], (size_t)words));
-          dirs_words[0] = words;
-        }
+        for (int c = 0; c < (pl.tune ? ncand : 1); ++c)
+          words = std::max(words, trace_scratch_words(G.Q, G.R, std::min(G.count, sub),
+                                                      pl.tune ? cg[c] : pl.g,
+                                                      pl.tune ? crpl[c] : pl.rpl));
+        packed_launches += (G.count + sub - 1) / sub;
+        packed_pairs += G.count;
+      }
+      if (words > dirs_words[0]) {
+        CK(sc.get(&dirs[0], (size_t)words));
+        dirs_words[0] = words;
+      }
+      auto trace_args = [&](size_t gi) {
+        const Group& G = groups[gi];
         FastArgs fa;
         memset(&fa, 0, sizeof(fa));
         fa.q = qbuf;
         fa.w = wbuf;
         fa.q_stride = q_stride;
         fa.w_stride = w_stride;
-        fa.Q = Q;
-        fa.R = R;
+        fa.Q = G.Q;
+        fa.R = G.R;
         fa.q_len = dql + c0;
         fa.r_len = drl + c0;
         fa.match = m;
         fa.mismatch = x;
         fa.gap_open = o;
         fa.gap_ext = e;
-        fa.bias = bias;
+        fa.bias = plans[gi].bias;
         fa.aln = aln;
         fa.best = best2;
         fa.dirs = dirs[0];
@@ -1995,18 +1989,29 @@ int swift_sw_pairs(swift_ctx* ctx, const char* qry, const int64_t* q_off, const 
         fa.qcons = cq;
         fa.rcons = cr;
         fa.cons_stride = cs;
-        fa.list = list;
+        fa.list = sorted + G.start;
         fa.count = gcount_d + gi;
-        if (tune) {
+        fa.shape_g = plans[gi].g;
+        fa.shape_rpl = plans[gi].rpl;
+        return fa;
+      };
+      for (size_t gi = 0; gi < groups.size(); ++gi) {
+        const Group& G = groups[gi];
+        if (G.gen) continue;
+        Plan& pl = plans[gi];
+        int32_t cg[16], crpl[16];
+        const int ncand = packed_shape_candidates(G.Q, cg, crpl, 16);
+        if (pl.tune) {
           // a sample from the middle of the class (its pairs are sorted by
-          // window length), each candidate warmed once and timed once
-          const int64_t ns = std::min<int64_t>(cnt, 16384);
+          // window length), each candidate launched once on a few of them
+          // (its code loaded) and timed once
+          const int64_t ns = std::min<int64_t>(G.count, 16384);
           int32_t* ns_d;
           CK(sc.get(&ns_d, 1));
           const int32_t ns32 = (int32_t)ns;
           CK(cudaMemcpyAsync(ns_d, &ns32, 4, cudaMemcpyHostToDevice, st));
-          FastArgs ta = fa;
-          ta.list = list + (cnt - ns) / 2;
+          FastArgs ta = trace_args(gi);
+          ta.list += (G.count - ns) / 2;
           ta.count = ns_d;
           ta.list_offset = 0;
           cudaEvent_t e0 = ctx->ev[9], e1 = ctx->ev[10];
@@ -2018,7 +2023,7 @@ int swift_sw_pairs(swift_ctx* ctx, const char* qry, const int64_t* q_off, const 
             float t = 0;
             for (int rep = 0; rep < 2; ++rep) {
               CK(cudaEventRecord(e0, st));
-              const int kk = launch_sw_trace(st, ta, ns);
+              const int kk = launch_sw_trace(st, ta, rep == 0 ? 32 : ns);
               if (kk == 0) return fail(ctx, SWIFT_E_DEVICE, "trace pass could not launch");
               launches += kk;
               CKLAUNCH();
@@ -2032,28 +2037,81 @@ int swift_sw_pairs(swift_ctx* ctx, const char* qry, const int64_t* q_off, const 
               best = c;
             }
           }
-          ctx->tuned[tkey] = {cg[best], crpl[best]};
-          sg = cg[best];
-          srpl = crpl[best];
+          ctx->tuned[(G.Q / 8) * 64 + (G.R + 63) / 64] = {cg[best], crpl[best]};
+          pl.g = cg[best];
+          pl.rpl = crpl[best];
         }
-        fa.shape_g = sg;
-        fa.shape_rpl = srpl;
-        {
-          int32_t dg[1], dr[1];
-          packed_shape_candidates(Q, dg, dr, 1);
-          const int pc = packed_class(Q);
-          if (pc >= 0 && pc < 8) {
-            ps.shape_lanes[pc] = sg ? sg : dg[0];
-            ps.shape_rows[pc] = sg ? srpl : dr[0];
-          }
+        const int pc = packed_class(G.Q);
+        if (pc >= 0 && pc < 8) {
+          ps.shape_lanes[pc] = pl.g ? pl.g : cg[0];
+          ps.shape_rows[pc] = pl.g ? pl.rpl : crpl[0];
         }
-        for (int64_t off = 0; off < cnt; off += sub) {
+      }
+      // The launches alternate between the context stream and the side
+      // stream, each with its own scratch, largest class first: a class is a
+      // few waves of warps, and its last one, and its walk, then share the
+      // GPU with the next class (650 K uneven pairs 10.5 -> 10.0 ms, 32 K 2.5 ->
+      // 1.7; with few classes merged 1.1).
+      bool two = packed_launches > 1 && packed_pairs >= kAlternatePairs;
+      if (two && words > dirs_words[1]) {
+        if (sc.get(&dirs[1], (size_t)words) == cudaSuccess) {
+          dirs_words[1] = words;
+        } else {
+          cudaGetLastError();  // no memory for it: one stream
+          two = false;
+        }
+      }
+      if (two) {
+        const int rc = side_fork(ctx);
+        if (rc != SWIFT_OK) return rc;
+        joined.armed = true;
+      }
+      int turn = 0;
+      for (size_t gr = groups.size(); gr-- > 0;) {
+        const Group& G = groups[gr];
+        if (G.gen) {
+          cudaStream_t bs = two && (turn++ & 1) ? ctx->side : st;
+          SwArgs sa;
+          memset(&sa, 0, sizeof(sa));
+          sa.q = qbuf;
+          sa.w = wbuf;
+          sa.q_stride = q_stride;
+          sa.w_stride = w_stride;
+          sa.Q = G.Q;
+          sa.R = G.R;
+          sa.match = m;
+          sa.mismatch = x;
+          sa.gap_open = o;
+          sa.gap_ext = e;
+          sa.n = G.count;
+          sa.aln = aln;
+          sa.qcons = cq;
+          sa.rcons = cr;
+          sa.cons_stride = cs;
+          sa.list = sorted + G.start;
+          sa.count = gcount_d + gr;
+          const int rc = launch_sw(bs, sa, &ctx->err);
+          if (rc != SWIFT_OK) return rc;
+          CKLAUNCH();
+          ++launches;
+          ps.generic_pairs += G.count;
+          continue;
+        }
+        FastArgs fa = trace_args(gr);
+        for (int64_t off = 0; off < G.count; off += sub) {
+          const int t = two ? turn++ & 1 : 0;
+          fa.dirs = dirs[t];
+          fa.dirs_words = dirs_words[t];
           fa.list_offset = off;
-          const int kk = launch_sw_trace(st, fa, std::min(sub, cnt - off));
+          const int kk = launch_sw_trace(t ? ctx->side : st, fa, std::min(sub, G.count - off));
           if (kk == 0) return fail(ctx, SWIFT_E_DEVICE, "trace pass could not launch");
           launches += kk;
           CKLAUNCH();
         }
+      }
+      if (joined.armed) {
+        const int rc = joined.join();
+        if (rc != SWIFT_OK) return rc;
       }
       // long pairs: one CTA each, largest first, in launches of many waves
       // (the block scheduler fills SMs freed by small pairs) whose direction

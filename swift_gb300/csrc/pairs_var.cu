@@ -64,18 +64,33 @@ __global__ void __launch_bounds__(kVarWarps * 32) pack_var_kernel(VarPairArgs a)
   char* qd = a.qbuf + i * a.q_stride;
   char* wd = a.wbuf + i * a.w_stride;
   bool odd = false, bad = false;
-  for (int t = lane; t < a.q_stride; t += 32) {
-    const char c = t < Q ? qs[t] : '\x01';
-    qd[t] = c;
-    if (t < Q && !acgt((uint8_t)c)) odd = true;
-    if (t < Q && (uint8_t)c < 2) bad = true;
-  }
-  for (int t = lane; t < a.w_stride; t += 32) {
-    const char c = t < R ? ws[t] : '\0';
-    wd[t] = c;
-    if (t < R && !acgt((uint8_t)c)) odd = true;
-    if (t < R && (uint8_t)c < 2) bad = true;
-  }
+  // len bytes of src (any alignment) to a row of `stride` bytes, four at a
+  // time, `fill` past them (strides are multiples of 16); the loads are words
+  // that hold a byte of [src, src + len)
+  auto row = [&](const char* src, int len, char* dst, int stride, uint32_t fill) {
+    const uintptr_t ad = (uintptr_t)src;
+    const uint32_t* wp = reinterpret_cast<const uint32_t*>(ad & ~(uintptr_t)3);
+    const int off = (int)(ad & 3);
+    for (int t = 4 * lane; t < stride; t += 128) {
+      uint32_t v = fill;
+      if (t < len) {
+        const uint32_t lo = wp[t >> 2];
+        const uint32_t hi = off && t + 4 - off < len ? wp[(t >> 2) + 1] : 0u;
+        const uint32_t x = __funnelshift_r(lo, hi, 8 * off);
+        const uint32_t keep = len - t >= 4 ? ~0u : (1u << (8 * (len - t))) - 1u;
+        // a byte outside ACGTacgt, and one below 2 (a zero byte of x with
+        // the lowest bits off)
+        const uint32_t c = ((x >> 1) ^ (x >> 2)) & 0x03030303u, n = c | (c >> 4);
+        odd |= ((__byte_perm(0x54474341u, 0u, (n & 0x33u) | ((n >> 8) & 0x3300u)) ^ x) & 0xDFDFDFDFu & keep) != 0u;
+        const uint32_t z = (x | ~keep) & 0xFEFEFEFEu;
+        bad |= ((z - 0x01010101u) & ~z & 0x80808080u) != 0u;
+        v = (x & keep) | (fill & ~keep);
+      }
+      *reinterpret_cast<uint32_t*>(dst + t) = v;
+    }
+  };
+  row(qs, Q, qd, (int)a.q_stride, 0x01010101u);
+  row(ws, R, wd, (int)a.w_stride, 0u);
   odd = __any_sync(0xffffffffu, odd);
   bad = __any_sync(0xffffffffu, bad);
   if (lane == 0 && bad) atomicOr(a.bad, 1u);

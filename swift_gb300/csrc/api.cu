@@ -948,8 +948,30 @@ int upload_reads(swift_ctx* ctx, const char* b, size_t len, swift_reads** out,
   CKR(cudaMemcpyAsync(r->d_bytes, b, len, cudaMemcpyHostToDevice, st));
   CKR(cudaEventRecord(ctx->ev[11], st));
   float copy_ms = 0;
-  {
-    Scratch sc(st);
+  ParseSummary h_sum = {INT32_MAX, 0, 0, 0};
+  unsigned long long h_err = ~0ull;
+  uint64_t n_lines = 0;
+  Scratch sc(st);
+  Readback rb(ctx);
+  auto alloc_reads = [&](uint64_t n) {
+    const size_t bytes = std::max<uint64_t>(n, 1) * sizeof(DevRead);
+    return transient ? cudaMallocAsync(&r->d_rd, bytes, st) : cudaMalloc(&r->d_rd, bytes);
+  };
+  if (len > 0 && len <= kParseSmall) {
+    ParseSmall* out_d;
+    uint64_t* nl;
+    CKR(sc.get(&out_d, 1));
+    CKR(sc.get(&nl, len));
+    CKR(alloc_reads(len / 2 + 1));
+    launch_parse_small(st, r->d_bytes, len, nl, r->d_rd, out_d, max_read);
+    CKR(cudaGetLastError());
+    ParseSmall h;
+    CKR(rb.get(&h, out_d, sizeof(h)));
+    CKR(rb.sync());
+    h_sum = h.sum;
+    h_err = h.err;
+    n_lines = h.n_lines;
+  } else {
     const uint64_t tiles = parse_tiles(len);
     uint32_t *cnt, *off, *n_nl_d;
     unsigned long long* err;
@@ -968,34 +990,30 @@ int upload_reads(swift_ctx* ctx, const char* b, size_t len, swift_reads** out,
     exclusive_scan_u32(st, cnt, off, (int64_t)tiles, tmp, n_nl_d);
     CKR(cudaGetLastError());
     uint32_t n_nl = 0;
-    Readback rb(ctx);
     CKR(rb.get(&n_nl, n_nl_d, 4));
     CKR(rb.sync());
-    CKR(cudaEventElapsedTime(&copy_ms, ctx->ev[10], ctx->ev[11]));
-    const uint64_t n_lines = n_nl + ((len > 0 && b[len - 1] != '\n') ? 1 : 0);
+    n_lines = n_nl + ((len > 0 && b[len - 1] != '\n') ? 1 : 0);
     uint64_t* nl;
     CKR(sc.get(&nl, std::max<uint64_t>(n_nl, 1)));
-    const size_t rd_bytes = std::max<uint64_t>(n_lines / 2, 1) * sizeof(DevRead);
-    CKR(transient ? cudaMallocAsync(&r->d_rd, rd_bytes, st) : cudaMalloc(&r->d_rd, rd_bytes));
+    CKR(alloc_reads(n_lines / 2));
     launch_parse_newlines(st, r->d_bytes, len, off, nl);
     launch_parse_lines(st, r->d_bytes, len, nl, n_nl, n_lines, r->d_rd, sum, err, max_read);
     CKR(cudaGetLastError());
-    unsigned long long h_err = 0;
-    ParseSummary h_sum;
     CKR(rb.get(&h_err, err, sizeof(h_err)));
     CKR(rb.get(&h_sum, sum, sizeof(h_sum)));
     CKR(rb.sync());
-    if (h_err != ~0ull) {
-      std::string m;
-      const int code = parse_error((uint32_t)(h_err & 0xFF), h_err >> 8, &m, max_read);
-      return bail(code, m);
-    }
-    r->n = (int64_t)(n_lines / 2);
-    r->n_gt = (int64_t)((n_lines + 1) / 2);  // '>' occurs only at header starts
-    r->first_len = h_sum.first_len;
-    r->min_len = r->n ? h_sum.min_len : 0;
-    r->max_len = h_sum.max_len;
   }
+  CKR(cudaEventElapsedTime(&copy_ms, ctx->ev[10], ctx->ev[11]));
+  if (h_err != ~0ull) {
+    std::string m;
+    const int code = parse_error((uint32_t)(h_err & 0xFF), h_err >> 8, &m, max_read);
+    return bail(code, m);
+  }
+  r->n = (int64_t)(n_lines / 2);
+  r->n_gt = (int64_t)((n_lines + 1) / 2);  // '>' occurs only at header starts
+  r->first_len = h_sum.first_len;
+  r->min_len = r->n ? h_sum.min_len : 0;
+  r->max_len = h_sum.max_len;
 #undef CKR
   r->repeats = phase1_stale_repeats(r->n, r->n_gt);
   if (h2d_ms) *h2d_ms = copy_ms;

@@ -285,6 +285,16 @@ enum : uint32_t {
 struct ParseSummary {
   int32_t min_len, max_len, first_len, pad;
 };
+// a whole file of 1 .. kParseSmall bytes by one block; nl has room for n
+// positions, rd for n / 2 + 1 reads
+constexpr uint64_t kParseSmall = 65536;
+struct ParseSmall {
+  ParseSummary sum;
+  unsigned long long err;     // ~0: none
+  uint64_t n_lines;
+};
+void launch_parse_small(cudaStream_t st, const char* b, uint64_t n, uint64_t* nl, DevRead* rd,
+                        ParseSmall* out, int max_read);
 unsigned parse_tiles(uint64_t n);
 void launch_parse_tiles(cudaStream_t st, const char* b, uint64_t n, uint32_t* cnt,
                         unsigned long long* err);

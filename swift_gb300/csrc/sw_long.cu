@@ -539,10 +539,12 @@ __global__ void __launch_bounds__(kLT, 2) sw_long16_kernel(LongArgs a) {
 // A walk is a chain of dependent reads.  The warp fetches a tile of 256
 // direction words at once: of the threads whose rows the walk passes next,
 // the steps around the diagonal from its cell (plus the query and window
-// bytes there); the moves then run from shared memory, every lane alike,
-// until one leaves the tile.  (One thread per pair read four words at a time,
-// and some walk of its warp waited for memory on almost every move: 4.2 ms
-// for queries of 3 to 4 kb, 0.9 ms now.)
+// bytes there).  Within the tile the lanes look at 32 cells of the diagonal
+// together, and a run of DIAG moves, most of an alignment, is one step of the
+// walk; gap moves go one by one.  (One thread per pair read four words at a
+// time, and some walk of its warp waited for memory on almost every move: 4.2
+// ms for queries of 3 to 4 kb; with tiles but move by move 0.9 ms, 110
+// instructions a move; LWALK_US us now.)
 constexpr int kTileWords = 256;
 constexpr int kTileSteps = 32;  // of a stream: 16 columns a diagonal crosses in it, 9
                                 // and more before them, about 5 past (gaps)
@@ -626,47 +628,73 @@ __global__ void __launch_bounds__(kWalkWarps * 32) sw_long_walk_kernel(LongArgs 
   char* rc = a.rcons ? a.rcons + (int64_t)p * a.cons_stride : nullptr;
   int d = (cr == 0 || cc == 0) ? kNone : dir_of(code(), h);
   int tick = -1, nref = -1, start = 0;
-  char my_q = 0, my_r = 0;  // the bytes of move tick with tick % 32 == lane
+  // the cell has moved to (cr, cc): its thread, row and lane
+  auto moved = [&]() {
+    const int tt = (cr - 1) / rpl;
+    m += t - tt;
+    t = tt;
+    k = (cr - 1) - t * rpl;
+    wl = lane_of(t, k);
+    if (m < kTileStreams) lo_m = lo[m];
+  };
   while (d != kNone) {
-    const bool up = d != kLeft, left = d != kUp;  // row / column move
-    const char qb = qs[rows0 - cr], rb = ws[cols0 - cc];
-    ++tick;
-    nref += left ? 1 : 0;
-    if (lane == (tick & 31)) {
-      my_r = left ? rb : '-';
-      my_q = up ? qb : '-';
+    if (d == kDiag) {
+      // A run of DIAG moves at once: lane i looks at the cell i moves on.
+      const int row = cr - lane, col = cc - lane;
+      bool diag = false, eq = false;
+      char qb = 0, rb = 0;
+      if (row >= 1 && col >= 1) {
+        const int tt = (row - 1) / rpl, kk = (row - 1) - tt * rpl, mm = m + t - tt;
+        const int step = col + lane_of(tt, kk) - 1;
+        if (mm < kTileStreams && (uint32_t)(step - lo[mm]) < (uint32_t)kTileSteps) {
+          const uint32_t word = tile[mm * kTileSteps + (step - lo[mm])];
+          const int sh = !P16 ? 2 * kk : kk >= half ? 16 + 2 * (rpl - 1 - kk) : 2 * (half - 1 - kk);
+          diag = ((word >> sh) & 3u) == (P16 ? 0u : 2u);
+          qb = qs[rows0 - row];
+          rb = ws[cols0 - col];
+          const int uq = upcase((uint8_t)qb), ur = upcase((uint8_t)rb);
+          eq = uq == ur || uq == 'N' || ur == 'N';
+        }
+      }
+      const uint32_t em = __ballot_sync(0xffffffffu, eq);
+      // the lane's cell before its own move (P16: a code of DIAG is NONE at 0)
+      const int e0 = __popc(em & ((1u << lane) - 1));
+      const int hl = h - ma * e0 - x * (lane - e0);
+      const uint32_t stop = ~__ballot_sync(0xffffffffu, diag && (!P16 || hl != 0));
+      const int r = stop ? __ffs(stop) - 1 : 32;  // at least 1: the cell itself
+      if (lane < r && qc) {
+        rc[tick + 1 + lane] = rb;
+        qc[tick + 1 + lane] = qb;
+      }
+      const int er = __popc(r == 32 ? em : em & ((1u << r) - 1));
+      h -= ma * er + x * (r - er);
+      tick += r;
+      nref += r;
+      cr -= r;
+      cc -= r;
+      start = cc + 1;
+      if (cr == 0 || cc == 0) break;
+      moved();
+      d = dir_of(code(), h);
+      continue;
     }
-    if ((tick & 31) == 31 && qc) {
-      rc[tick - 31 + lane] = my_r;
-      qc[tick - 31 + lane] = my_q;
+    // a gap move
+    const bool up = d == kUp;
+    ++tick;
+    nref += up ? 0 : 1;
+    if (lane == 0 && qc) {
+      rc[tick] = up ? '-' : ws[cols0 - cc];
+      qc[tick] = up ? qs[rows0 - cr] : '-';
     }
     start = cc;
     cr -= up ? 1 : 0;
-    cc -= left ? 1 : 0;
+    cc -= up ? 0 : 1;
     if (cr == 0 || cc == 0) break;
-    if (up) {
-      if (--k < 0) {
-        k = rpl - 1;
-        --t;
-        wl = lane_of(t, k);
-        if (++m < kTileStreams) lo_m = lo[m];
-      } else if (P16 && k == half - 1) {
-        --wl;
-      }
-    }
+    if (up) moved();
     const uint32_t pc = code();
-    if (d == kDiag) {
-      const int uq = upcase((uint8_t)qb), ur = upcase((uint8_t)rb);
-      h -= (uq == ur || uq == 'N' || ur == 'N') ? ma : x;
-    } else {
-      // the gap costs gap_ext when the predecessor itself moved the same way
-      h -= (d == kUp ? pc == kUpCode : pc == kLeftCode) ? e : o;
-    }
+    // it costs gap_ext when the predecessor itself moved the same way
+    h -= (up ? pc == kUpCode : pc == kLeftCode) ? e : o;
     d = dir_of(pc, h);
-  }
-  if (qc && tick >= 0 && lane <= (tick & 31) && (tick & 31) != 31) {
-    rc[(tick & ~31) + lane] = my_r;
-    qc[(tick & ~31) + lane] = my_q;
   }
   if (lane == 0) {
     DevAln out;

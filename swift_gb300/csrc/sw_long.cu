@@ -544,7 +544,7 @@ __global__ void __launch_bounds__(kLT, 2) sw_long16_kernel(LongArgs a) {
 // walk; gap moves go one by one.  (One thread per pair read four words at a
 // time, and some walk of its warp waited for memory on almost every move: 4.2
 // ms for queries of 3 to 4 kb; with tiles but move by move 0.9 ms, 110
-// instructions a move; LWALK_US us now.)
+// instructions a move; 0.15 ms now.)
 constexpr int kTileWords = 256;
 constexpr int kTileSteps = 32;  // of a stream: 16 columns a diagonal crosses in it, 9
                                 // and more before them, about 5 past (gaps)

@@ -95,7 +95,7 @@ int launch_shape(cudaStream_t st, const FastArgs& a, int64_t max_pairs) {
 int launch_walk(cudaStream_t st, const FastArgs& a, int64_t max_pairs) {
   const Shape s = shape_of(a);
   if (s.G == 0 || max_pairs <= 0) return 0;
-  const unsigned grid = (unsigned)((max_pairs + kWalkThreads - 1) / kWalkThreads);
+  const unsigned grid = (unsigned)((max_pairs + kWalkThreads / 32 - 1) / (kWalkThreads / 32));
 #define SWIFT_WK(G_, R_)                                      \
   if (s.G == G_ && s.RPL == R_) {                              \
     sw_walk_kernel<G_, R_><<<grid, kWalkThreads, 0, st>>>(a);  \
@@ -194,8 +194,6 @@ int launch_sw_score(cudaStream_t st, const FastArgs& a, int64_t max_pairs) {
 
 int launch_sw_trace(cudaStream_t st, const FastArgs& a, int64_t max_pairs, cudaEvent_t before,
                     cudaEvent_t after) {
-  // the walk stores 32-bit words, and reads words of the query and window rows
-  if (a.cons_stride % 4 != 0 || (a.q_stride | a.w_stride) % 4 != 0) return 0;
   if (trace_scratch_words(a.Q, a.R, max_pairs, a.shape_g, a.shape_rpl) > a.dirs_words) return 0;
   FastArgs b = a;
   b.chunk = max_pairs;

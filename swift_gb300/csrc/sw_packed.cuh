@@ -496,62 +496,40 @@ __global__ void __launch_bounds__(kPkWarps * 32, (TRACE || RPL > 13) ? 16 / kPkW
   if (warp * kPairs < nlist) packed_item<G, RPL, TRACE, VAR>(a, warp, nlist, wsel_all, wib, lane);
 }
 
-// Traceback walk (src/smithWaterman.cu:911-1026), one thread per printed
-// pair over the 2-bit directions the trace pass streamed out.
+// Traceback walk (src/smithWaterman.cu:911-1026), one warp per printed pair
+// over the 2-bit directions the trace pass streamed out.
 //
-// Each move depends on the one before, so a walk is bound by the latency of
-// its loads.  A warp's walks refill together: a round copies into shared
-// memory everything the next kWalkMoves moves of a walk can touch (the last
-// kWalkMoves + 1 steps of its lane's direction stream and of the streams of
-// the lanes above that it can reach, the query and window bytes before its
-// cell), all of it loads that do not wait for one another, and the moves then
-// run from shared memory.  (With each walk refilling a register cache when it
-// left it, some walk of a warp waited for memory on almost every move: 10,000
-// reads' walks took 125 us, with rounds 51 us; more moves a round load more
-// than the walks use.)
-constexpr int kWalkThreads = 128;  // small blocks: walks of uneven length leave SMs sooner
-constexpr int kWalkMoves = 8;
-
-template <int G, int RPL>
-struct WalkRound {
-  static constexpr int kNW = DirLayout<RPL>::kWords;
-  static constexpr int kStreams = (kWalkMoves + RPL - 1) / RPL + 1;
-  // 16-byte blocks of a stream: its words and up to 3 before them
-  static constexpr int kBlocks = ((kWalkMoves + 1) * kNW + 3 + 3) / 4;
-  static constexpr int kSeq = (kWalkMoves + 3 + 3) / 4;  // words of query or window bytes
-  static constexpr int kWordsAll = kStreams * kBlocks * 4 + 2 * kSeq;
-};
+// Most moves of an alignment are DIAG.  A round looks at the walk's cell and
+// the 31 after it on its diagonal, one per lane: the lanes load their words
+// (a lane's stream holds them side by side) and bytes without waiting for one
+// another, ballots give how far the moves stay DIAG and how many of them
+// match, and the lanes write their bytes of the strings; a gap move ends the
+// round.  So a walk waits for memory every 32 moves or gap, where a thread
+// per pair waited every 8 moves (and before that on almost every one):
+// 10,000 reads' walks 51 -> 13 us, a million reads' 0.36 -> 0.18 ms.
+constexpr int kWalkThreads = 128;
 
 template <int G, int RPL>
 __global__ void __launch_bounds__(kWalkThreads) sw_walk_kernel(FastArgs a) {
-  using Round = WalkRound<G, RPL>;
   constexpr int kGroups = 32 / G;
   constexpr int kPairs = 2 * kGroups;
-  constexpr int kNW = Round::kNW;
-  // [word][thread]: a thread's words never share a bank with another's
-  __shared__ uint32_t sh[Round::kWordsAll * kWalkThreads];
+  constexpr int kNW = DirLayout<RPL>::kWords;
+  const int lane = threadIdx.x & 31;
   const int64_t nlist = *a.count - a.list_offset;
-  const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= nlist || idx >= a.chunk) return;  // (no block-wide synchronisation below)
+  const int64_t idx = ((int64_t)blockIdx.x * kWalkThreads + threadIdx.x) >> 5;
+  if (idx >= nlist || idx >= a.chunk) return;  // (a whole warp)
   const int32_t p = a.list[a.list_offset + idx];
   const int64_t warp = idx / kPairs;
   const int g = (int)((idx % kPairs) >> 1);
-  const int hp = (int)(idx & 1);
-  const int R = a.R;
-  const int S8 = steps8(R, G);
+  const int shift_half = 16 * (int)(idx & 1);
+  const int S8 = steps8(a.R, G);
   const uint32_t* dirs = a.dirs + (warp * kGroups + g) * (int64_t)G * kNW * S8;
   const char* qg = a.q + (int64_t)p * a.q_stride;
   const char* wg = a.w + (int64_t)p * a.w_stride;
-  const int W = (a.r_len ? a.r_len[p] : R) + 1;  // the pair's own window for cell indices
-  const int shift_half = 16 * hp;
-  uint32_t* mine = sh + threadIdx.x;
-  const char* bytes = reinterpret_cast<const char*>(mine + Round::kStreams * Round::kBlocks * 4 * kWalkThreads);
-  // consensus bytes are gathered four at a time and stored as words
+  const int W = (a.r_len ? a.r_len[p] : a.R) + 1;  // the pair's own window for cell indices
   // (consensus strings are optional: coordinates only when qcons is null)
-  const bool cons = a.qcons != nullptr;
-  uint32_t* qcw = cons ? reinterpret_cast<uint32_t*>(a.qcons + (int64_t)p * a.cons_stride) : nullptr;
-  uint32_t* rcw = cons ? reinterpret_cast<uint32_t*>(a.rcons + (int64_t)p * a.cons_stride) : nullptr;
-  uint32_t qacc = 0, racc = 0;
+  char* qc = a.qcons ? a.qcons + (int64_t)p * a.cons_stride : nullptr;
+  char* rc = a.rcons ? a.rcons + (int64_t)p * a.cons_stride : nullptr;
   // Directions of the reference's kernel (NONE, DIAG, UP, LEFT) from the
   // 2-bit codes and the cell's score h, which the walk carries: a cell
   // with code 0 is NONE exactly when h = 0 (any other cell has h > 0).
@@ -559,125 +537,82 @@ __global__ void __launch_bounds__(kWalkThreads) sw_walk_kernel(FastArgs a) {
   auto dir_of = [](uint32_t code, int h) -> int {
     return code == 2u ? kUp : code == 1u ? kLeft : (h == 0 ? kNone : kDiag);
   };
-  const int m = a.match, x = a.mismatch, o = a.gap_open, e = a.gap_ext;
   auto upc = [](char c) -> char { return (unsigned)(c - 'a') < 26u ? (char)(c - 32) : c; };
+  const int m = a.match, x = a.mismatch, o = a.gap_open, e = a.gap_ext;
   const int2 b = a.best[p];
   int cr = b.y / W, cc = b.y % W;  // current cell
   int h = b.x;                     // its score
-  // its lane and row in the lane (kept as the walk moves up)
-  int ln = cr > 0 ? (cr - 1) / RPL : 0, k = cr > 0 ? (cr - 1) % RPL : 0;
-  int d = (cr == 0 || cc == 0) ? kNone : kDiag;  // the first round reads the cell's own
-  bool fresh = true;
   int tick = -1, nref = -1, start = 0;
-  while (d != kNone) {
-    // the round's words: stream t holds lane ln - t from word base(t) on
-    const int ln0 = ln, step_lo = cc - kWalkMoves + ln - 1;  // lane ln's earliest step
-    auto base = [&](int t) -> int {
-      const int lane0 = (ln0 - t) * S8, lo = step_lo - t;
-      return ((lane0 + max(lo, 0)) * kNW) & ~3;
-    };
-#pragma unroll
-    for (int t = 0; t < Round::kStreams; ++t) {
-      if (ln0 - t >= 0) {
-        const uint4* src = reinterpret_cast<const uint4*>(dirs + base(t));
-        uint4 v[Round::kBlocks];
-        // (blocks past a stream's last step lie in the next lane's stream or
-        // the scratch's spare groups)
-#pragma unroll
-        for (int q = 0; q < Round::kBlocks; ++q) v[q] = __ldg(src + q);
-#pragma unroll
-        for (int q = 0; q < Round::kBlocks; ++q) {
-          uint32_t* to = mine + (t * Round::kBlocks + q) * 4 * kWalkThreads;
-          to[0] = v[q].x;
-          to[kWalkThreads] = v[q].y;
-          to[2 * kWalkThreads] = v[q].z;
-          to[3 * kWalkThreads] = v[q].w;
-        }
-      }
+  int gap = kNone;                 // the gap move that led here, its cost still open
+  while (cr > 0 && cc > 0) {
+    // lane i: the cell i moves on along the diagonal
+    const int row = cr - lane, col = cc - lane;
+    const bool in = row >= 1 && col >= 1;
+    uint32_t code = 3u;
+    char qb = 0, rb = 0;
+    if (in) {
+      const int ln = (row - 1) / RPL, k = (row - 1) - ln * RPL;
+      const uint32_t word = __ldg(dirs + (ln * S8 + (col + ln - 1)) * kNW + (k >> 3));
+      qb = qg[row - 1];
+      rb = wg[col - 1];
+      const int last = kNW == 1 || k >= 8 ? RPL - 1 : 7;  // a word's rows, the last lowest
+      code = (word >> (shift_half + 2 * (last - k))) & 3u;
     }
-    // query rows and window columns before the cell, from 4-byte words (rows
-    // of the buffers start 16-byte aligned)
-    const int q0 = max(cr - kWalkMoves, 0) & ~3, w0 = max(cc - kWalkMoves, 0) & ~3;
-    {
-      const uint32_t* qs = reinterpret_cast<const uint32_t*>(qg + q0);
-      const uint32_t* ws = reinterpret_cast<const uint32_t*>(wg + w0);
-      uint32_t* to = mine + Round::kStreams * Round::kBlocks * 4 * kWalkThreads;
-#pragma unroll
-      for (int q = 0; q < Round::kSeq; ++q) {
-        // (words past the cell's are not needed and may lie past the row)
-        to[q * kWalkThreads] = q0 + 4 * q < cr ? __ldg(qs + q) : 0u;
-        to[(Round::kSeq + q) * kWalkThreads] = w0 + 4 * q < cc ? __ldg(ws + q) : 0u;
+    uint32_t c = __shfl_sync(0xffffffffu, code, 0);
+    // a gap costs gap_ext when its predecessor itself moved the same way
+    if (gap != kNone) h -= (gap == kUp ? c == 2u : c == 1u) ? e : o;
+    gap = kNone;
+    int d = dir_of(c, h);
+    if (d == kNone) break;
+    int at = 0;  // the lane of the current cell
+    if (d == kDiag) {
+      // the moves from lane 0 on that stay DIAG (a code of 0 is NONE where
+      // the score is 0)
+      const char uq = upc(qb), ur = upc(rb);
+      const uint32_t em = __ballot_sync(0xffffffffu, in && (uq == ur || uq == 'N' || ur == 'N'));
+      const int e0 = __popc(em & ((1u << lane) - 1));
+      const int hl = h - m * e0 - x * (lane - e0);
+      const uint32_t stop = ~__ballot_sync(0xffffffffu, in && code == 0u && hl != 0);
+      const int r = stop ? __ffs(stop) - 1 : 32;  // at least 1
+      if (lane < r && qc) {
+        rc[tick + 1 + lane] = rb;
+        qc[tick + 1 + lane] = qb;
       }
+      const int er = __popc(r == 32 ? em : em & ((1u << r) - 1));
+      h -= m * er + x * (r - er);
+      tick += r;
+      nref += r;
+      cr -= r;
+      cc -= r;
+      start = cc + 1;
+      if (r == 32 || cr == 0 || cc == 0) continue;
+      at = r;
+      c = __shfl_sync(0xffffffffu, code, at);
+      d = dir_of(c, h);
+      if (d == kNone) break;
     }
-    auto byte_at = [&](int w, int i) -> char {
-      return bytes[(w + (i >> 2)) * 4 * kWalkThreads + (i & 3)];
-    };
-    // the 2-bit code (2 UP, 1 LEFT, 0 DIAG or NONE) of the cell in lane l's
-    // row kk and column jj
-    auto code_at = [&](int l, int kk, int jj) -> uint32_t {
-      const int t = ln0 - l;
-      const int at = (l * S8 + (jj + l - 1)) * kNW + (kk >> 3) - base(t);
-      const uint32_t word = mine[(t * Round::kBlocks * 4 + at) * kWalkThreads];
-      const int rows_w = min(8, RPL - (kk & ~7));  // rows of the word, the last lowest
-      return (word >> (shift_half + 2 * (rows_w - 1 - (kk & 7)))) & 3u;
-    };
-    if (fresh) {
-      d = dir_of(code_at(ln, k, cc), h);
-      fresh = false;
+    // a gap move (its byte, '-' where the row or column stays)
+    const bool up = d == kUp;
+    const char gq = (char)__shfl_sync(0xffffffffu, (int)qb, at), gr = (char)__shfl_sync(0xffffffffu, (int)rb, at);
+    ++tick;
+    nref += up ? 0 : 1;
+    if (lane == 0 && qc) {
+      rc[tick] = up ? '-' : gr;
+      qc[tick] = up ? gq : '-';
     }
-    // One move per step: its consensus bytes (a gap where the row or column
-    // stays), then, unless it reached row or column 0, the predecessor's
-    // score (the substitution score for a DIAG move; for a gap, gap_ext when
-    // the predecessor itself moved the same way, else gap_open) and
-    // direction.  The walk ends at a NONE cell or at the border.
-    for (int mv = 0; mv < kWalkMoves && d != kNone; ++mv) {
-      const bool up = d != kLeft, left = d != kUp;  // row / column move
-      const char qc = byte_at(0, cr - 1 - q0), rc = byte_at(Round::kSeq, cc - 1 - w0);
-      ++tick;
-      nref += left ? 1 : 0;
-      {
-        const int sh8 = 8 * (tick & 3);
-        racc |= (uint32_t)(uint8_t)(left ? rc : '-') << sh8;
-        qacc |= (uint32_t)(uint8_t)(up ? qc : '-') << sh8;
-        if ((tick & 3) == 3) {
-          if (cons) {
-            rcw[tick >> 2] = racc;
-            qcw[tick >> 2] = qacc;
-          }
-          racc = qacc = 0;
-        }
-      }
-      start = cc;
-      cr -= up ? 1 : 0;
-      cc -= left ? 1 : 0;
-      if (cr == 0 || cc == 0) {
-        d = kNone;
-        break;
-      }
-      if (up && --k < 0) {
-        k = RPL - 1;
-        --ln;
-      }
-      const uint32_t pc = code_at(ln, k, cc);
-      if (d == kDiag) {
-        const char uq = upc(qc), ur = upc(rc);
-        h -= (uq == ur || uq == 'N' || ur == 'N') ? m : x;
-      } else {
-        h -= (d == kUp ? pc == 2u : pc == 1u) ? e : o;
-      }
-      d = dir_of(pc, h);
-    }
+    start = cc;
+    cr -= up ? 1 : 0;
+    cc -= up ? 0 : 1;
+    gap = d;
   }
-  if (cons && tick >= 0 && (tick & 3) != 3) {
-    rcw[tick >> 2] = racc;
-    qcw[tick >> 2] = qacc;
+  if (lane == 0) {
+    DevAln out;
+    out.score = b.x;
+    out.start = start;
+    out.end = start + nref;
+    out.len = tick + 1;
+    a.aln[p] = out;
   }
-  DevAln out;
-  out.score = b.x;
-  out.start = start;
-  out.end = start + nref;
-  out.len = tick + 1;
-  a.aln[p] = out;
 }
 
 }  // namespace

@@ -40,6 +40,12 @@ __device__ bool names_equal(const FormatArgs& a, const DevPair& s, const DevPair
   // which the comparison below finds equal whenever the name and its '*'
   // fit the slot
   if (s.read == t.read && a.rd[s.read].name_len + 1 < kNameMax) return true;
+  // names as long as one another (no byte of a name is 0) that end otherwise:
+  // most neighbours, whose numbers at the end differ
+  const DevRead &u = a.rd[s.read], &v = a.rd[t.read];
+  if (u.name_len == v.name_len && u.name_len > 0 && u.name_len < kNameMax &&
+      a.reads[u.name_off + u.name_len] != a.reads[v.name_off + v.name_len])
+    return false;
   // qryNameCmp over the 50-byte name slots
   int i;
   for (i = 0; i < kNameMax; ++i) {
@@ -57,7 +63,10 @@ __device__ bool names_equal(const FormatArgs& a, const DevPair& s, const DevPair
 // Record j opens a Phase-2 batch: every a.batch records, or where the wave's
 // per-request flags say so.
 __device__ __forceinline__ bool opens_batch(const FormatArgs& a, int64_t j) {
-  return a.batch_start ? a.batch_start[j] != 0 : j % a.batch == 0;
+  if (a.batch_start) return a.batch_start[j] != 0;
+  // (a 64-bit remainder takes a hundred instructions)
+  return a.n <= UINT32_MAX && a.batch <= UINT32_MAX ? (uint32_t)j % (uint32_t)a.batch == 0
+                                                    : j % a.batch == 0;
 }
 // last record of the best-per-read group that starts at j
 __device__ __forceinline__ int64_t group_end(const FormatArgs& a, int64_t j) {
@@ -86,19 +95,54 @@ __global__ void select_kernel(FormatArgs a) {
 // record, and settled one at least.  Its unsettled records score at most its
 // bound, below every settled one, so the group's pick is its first largest
 // settled score.  The other groups are left open, whole.
+// A warp looks at 32 records at once, each lane compares its record's name
+// with the one before: the groups that end within the warp are lanes between
+// two heads, their largest score a few shuffles.  A group that runs past the
+// warp's records is its first thread's, in a loop.  (With a thread per group
+// in that loop throughout, and an addition per warp, 4.13 M records took 206 us;
+// 94 now.)
 __global__ void settle_kernel(FormatArgs a, const uint8_t* __restrict__ state, uint32_t* open,
                               uint8_t* group_start, int32_t* n_settled) {
   const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int lane = threadIdx.x & 31;
+  const bool in = j < a.n;
+  // (the score before it is known to be wanted: one wait for memory less)
+  const uint8_t s = in ? state[j] : 0;
+  const int seen = in ? a.aln[j].score : 0;
+  // (lanes past the last record are heads: they end its group)
+  const bool head = !in || opens_batch(a, j) || !names_equal(a, a.pairs[j], a.pairs[j - 1]);
+  const int score = s == kGaplessDone ? seen : 0;
+  const uint32_t heads = __ballot_sync(0xffffffffu, head);
+  const uint32_t others = __ballot_sync(0xffffffffu, in && s == kGaplessOther);
+  const uint32_t upto = heads & (0xffffffffu >> (31 - lane));   // this lane and before
+  const uint32_t after = heads & ~(0xffffffffu >> (31 - lane));
+  const int first = upto ? 31 - __clz(upto) : 0;
+  const int next = after ? __ffs(after) - 1 : 0;  // 0: past the warp
+  // the largest score, and of its lanes the first, of the group from this lane on
+  int best = score > 0 ? (score << 5) | (31 - lane) : 0;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const int o = __shfl_down_sync(0xffffffffu, best, d);
+    if (lane + d < next) best = max(best, o);
+  }
+  best = __shfl_sync(0xffffffffu, best, first);
   int settled = 0;
-  if (j < a.n && (opens_batch(a, j) || !names_equal(a, a.pairs[j], a.pairs[j - 1]))) {
+  if (in && upto && next) {
+    const uint32_t group = ((1u << next) - 1) & ~((1u << first) - 1);
+    const int pick = best > 0 && !(others & group) ? 31 - (best & 31) : -1;
+    a.keep[j] = lane == pick ? 1 : 0;
+    open[j] = pick < 0 ? 1u : 0u;
+    group_start[j] = head ? 1 : 0;
+    if (head && pick >= 0) settled = next - first;
+  } else if (in && head) {
     const int64_t e = group_end(a, j);
     int64_t pick = -1;
     int mx = 0;
     bool known = true;
     for (int64_t i = j; i <= e; ++i) {
-      const uint8_t s = state[i];
-      known = known && s != kGaplessOther;
-      if (s == kGaplessDone && a.aln[i].score > mx) {
+      const uint8_t si = state[i];
+      known = known && si != kGaplessOther;
+      if (si == kGaplessDone && a.aln[i].score > mx) {
         mx = a.aln[i].score;
         pick = i;
       }
@@ -111,9 +155,18 @@ __global__ void settle_kernel(FormatArgs a, const uint8_t* __restrict__ state, u
     }
     if (pick >= 0) settled = (int)(e - j + 1);
   }
-  block_count(settled > 0, n_settled + 1);
+  // one addition per block: a warp's each to the same address took most of
+  // the kernel's time
+  __shared__ int32_t sum;
+  if (threadIdx.x == 0) sum = 0;
+  const int32_t groups = __syncthreads_count(settled > 0);
   settled = __reduce_add_sync(0xffffffffu, settled);
-  if ((threadIdx.x & 31) == 0 && settled) atomicAdd(n_settled, settled);
+  if (lane == 0 && settled) atomicAdd(&sum, settled);
+  __syncthreads();
+  if (threadIdx.x == 0 && sum) {
+    atomicAdd(n_settled, sum);
+    atomicAdd(n_settled + 1, groups);
+  }
 }
 
 __global__ void open_kernel(const uint8_t* __restrict__ state, int64_t n, uint32_t* open) {
@@ -509,7 +562,7 @@ void launch_select(cudaStream_t st, const FormatArgs& a) {
 void launch_settle(cudaStream_t st, const FormatArgs& a, const uint8_t* state, uint32_t* open,
                    uint8_t* group_start, int32_t* n_settled) {
   if (a.n <= 0) return;
-  settle_kernel<<<(unsigned)((a.n + 255) / 256), 256, 0, st>>>(a, state, open, group_start, n_settled);
+  settle_kernel<<<(unsigned)((a.n + 511) / 512), 512, 0, st>>>(a, state, open, group_start, n_settled);
 }
 
 void launch_open(cudaStream_t st, const uint8_t* state, int64_t n, uint32_t* open) {

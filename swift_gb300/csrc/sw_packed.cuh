@@ -8,9 +8,9 @@
 //                stopped once the score is settled or provably too low to
 //                be picked);
 //   trace pass   (TRACE = true):  for the printed pairs, the first
-//                row-major maximum and 4-bit directions streamed to global
+//                row-major maximum and 2-bit directions streamed to global
 //                scratch; sw_walk_kernel then walks the reference's
-//                traceback, one thread per pair.
+//                traceback, one warp per pair.
 //
 // Encoding.  Each cell is kept as Hx = 16*H + code + B, where code is the
 // one-hot direction the reference would store (NONE 8, DIAG 4, UP 2,

@@ -1485,28 +1485,22 @@ int swift_sw_batch(swift_ctx* ctx, const char* qry, const char* ref, int32_t Q, 
   const int64_t chunk = std::min<int64_t>(n, 131072);
   BatchArgs ba;
   FastArgs fa;
-  BatchOutArgs bo;
   int32_t* counts = nullptr;
   memset(&ba, 0, sizeof(ba));
   memset(&fa, 0, sizeof(fa));
-  memset(&bo, 0, sizeof(bo));
   if (packed) {
     ba.Q = Q;
     ba.R = R;
     ba.q_stride = ((int64_t)Q + 16) & ~(int64_t)15;
     ba.w_stride = ((int64_t)R + 16) & ~(int64_t)15;
-    fa.cons_stride = (cs + 15) & ~(int64_t)15;  // the walk stores words
     few_pairs_shape(Q, chunk, &fa.shape_g, &fa.shape_rpl);
     fa.dirs_words = trace_scratch_words(Q, R, chunk, fa.shape_g, fa.shape_rpl);
     packed = sc.get(&ba.qbuf, (size_t)(chunk * ba.q_stride)) == cudaSuccess &&
              sc.get(&ba.wbuf, (size_t)(chunk * ba.w_stride)) == cudaSuccess &&
              sc.get(&ba.fast, (size_t)chunk) == cudaSuccess &&
              sc.get(&ba.gen, (size_t)chunk) == cudaSuccess &&
-             sc.get(&ba.packed, (size_t)chunk) == cudaSuccess &&
              sc.get(&counts, 2) == cudaSuccess &&
              sc.get(&fa.best, (size_t)chunk) == cudaSuccess &&
-             sc.get(&fa.qcons, (size_t)(chunk * fa.cons_stride)) == cudaSuccess &&
-             sc.get(&fa.rcons, (size_t)(chunk * fa.cons_stride)) == cudaSuccess &&
              sc.get(&fa.dirs, (size_t)fa.dirs_words) == cudaSuccess;
     if (!packed) cudaGetLastError();  // no memory for it: the int32 kernel
   }
@@ -1560,6 +1554,9 @@ int swift_sw_batch(swift_ctx* ctx, const char* qry, const char* ref, int32_t Q, 
     fa.gap_ext = e;
     fa.bias = bias;
     fa.aln = aln;
+    fa.qcons = a.qcons;  // (the walk writes bytes: rows of any stride)
+    fa.rcons = a.rcons;
+    fa.cons_stride = cs;
     fa.list = ba.fast;
     fa.count = ba.n_fast;
     if (launch_sw_trace(st, fa, cn) == 0)
@@ -1567,20 +1564,8 @@ int swift_sw_batch(swift_ctx* ctx, const char* qry, const char* ref, int32_t Q, 
     CKLAUNCH();
     rc = generic.join();
     if (rc != SWIFT_OK) return rc;
-    bo.n = cn;
-    bo.aln = aln;
-    bo.packed = ba.packed;
-    bo.score = dscore + c0;
-    bo.start = dstart + c0;
-    bo.end = dend + c0;
-    bo.len = dlen + c0;
-    bo.qfrom = fa.qcons;
-    bo.rfrom = fa.rcons;
-    bo.from_stride = fa.cons_stride;
-    bo.qto = a.qcons;
-    bo.rto = a.rcons;
-    bo.to_stride = cs;
-    launch_batch_out(st, bo);
+    aln_to_ref_layout_kernel<<<(unsigned)((cn + 255) / 256), 256, 0, st>>>(
+        aln, cn, dscore + c0, dstart + c0, dend + c0, dlen + c0);
     CKLAUNCH();
   }
   if (!out_dev) {

@@ -1,8 +1,8 @@
 // swift_sw_batch on the packed 16-bit passes: its pairs, any bytes at any
-// alignment, laid out in 16-byte rows and split by their bytes; and the
-// results taken back to the caller's layout.  Both kernels move each pair's
-// bytes once, a warp per pair (20,000 pairs of 100 x 300: 12 and 14 us beside
-// 222 us of trace pass and 57 of walk; the int32 kernel 1.23 ms before).
+// alignment, laid out in 16-byte rows and split by their bytes.  Each pair's
+// bytes are moved once, by a warp (20,000 pairs of 100 x 300: 12 us beside 204
+// us of trace pass and 21 of walk, which writes the strings where the caller
+// wants them; the int32 kernel took 1.23 ms).
 #include "internal.h"
 
 namespace swift {
@@ -51,10 +51,7 @@ __global__ void __launch_bounds__(kBatchWarps * 32) pack_batch_kernel(BatchArgs 
     ok &= row(a.w + i * (a.R + 1), a.R, a.wbuf + i * a.w_stride, (int)a.w_stride, lane);
   }
   ok = __all_sync(0xffffffffu, ok);
-  if (lane == 0) {
-    plain[wib] = ok;
-    if (i < a.n) a.packed[i] = ok ? 1 : 0;
-  }
+  if (lane == 0) plain[wib] = ok;
   __syncthreads();
   const int t = threadIdx.x;
   const bool in = t < kBatchWarps && i0 + t < a.n;
@@ -62,34 +59,11 @@ __global__ void __launch_bounds__(kBatchWarps * 32) pack_batch_kernel(BatchArgs 
   block_append(in && !plain[t], (int32_t)(i0 + t), a.gen, a.n_gen);
 }
 
-__global__ void __launch_bounds__(kBatchWarps * 32) batch_out_kernel(BatchOutArgs a) {
-  const int lane = threadIdx.x & 31;
-  const int64_t i = (int64_t)blockIdx.x * kBatchWarps + (threadIdx.x >> 5);
-  if (i >= a.n) return;
-  const DevAln al = a.aln[i];
-  if (lane == 0) a.score[i] = (float)al.score;
-  if (lane == 1) a.start[i] = al.start;
-  if (lane == 2) a.end[i] = al.end;
-  if (lane == 3) a.len[i] = al.len;
-  if (!a.packed[i]) return;
-  const char *q = a.qfrom + i * a.from_stride, *r = a.rfrom + i * a.from_stride;
-  char *qt = a.qto + i * a.to_stride, *rt = a.rto + i * a.to_stride;
-  for (int z = lane; z < al.len; z += 32) {
-    qt[z] = q[z];
-    rt[z] = r[z];
-  }
-}
-
 }  // namespace
 
 void launch_pack_batch(cudaStream_t st, const BatchArgs& a) {
   if (a.n <= 0) return;
   pack_batch_kernel<<<(unsigned)((a.n + kBatchWarps - 1) / kBatchWarps), kBatchWarps * 32, 0, st>>>(a);
-}
-
-void launch_batch_out(cudaStream_t st, const BatchOutArgs& a) {
-  if (a.n <= 0) return;
-  batch_out_kernel<<<(unsigned)((a.n + kBatchWarps - 1) / kBatchWarps), kBatchWarps * 32, 0, st>>>(a);
 }
 
 }  // namespace swift

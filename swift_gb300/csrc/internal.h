@@ -483,23 +483,8 @@ struct BatchArgs {
   int64_t q_stride, w_stride;
   int32_t *fast, *n_fast;     // out: pairs of A, C, G, T bytes (either case) only,
   int32_t *gen, *n_gen;       // and the others
-  uint8_t* packed;            // out, per pair: 1 in the fast list
 };
 void launch_pack_batch(cudaStream_t st, const BatchArgs& a);
-// results in the caller's layout; the strings (stride to_stride, any
-// alignment) copied from from_stride rows where packed is set
-struct BatchOutArgs {
-  int64_t n;
-  const DevAln* aln;
-  const uint8_t* packed;
-  float* score;
-  int32_t *start, *end, *len;
-  const char *qfrom, *rfrom;
-  int64_t from_stride;
-  char *qto, *rto;
-  int64_t to_stride;
-};
-void launch_batch_out(cudaStream_t st, const BatchOutArgs& a);
 
 // pairs_var.cu: explicit pairs of varying lengths, sorted by shape
 constexpr uint32_t kVarKeys = 1u << 21;  // shape keys: generic bit, Q (9 bits), R (11 bits)

@@ -405,16 +405,23 @@ __global__ void aln_to_ref_layout_kernel(const DevAln* __restrict__ aln, int64_t
 // costs less than the passes, lists and host round trips that would spare
 // most of them: at these sizes each pass lasts as long as one pair does.
 constexpr int64_t kDirectPairs = 3072;
-// At most this many pairs all run on the int32 kernel: its warp a pair holds
-// directions in shared memory and walks them there, so at 1,024 pairs it ends
-// before the packed trace pass and walk, two launches of a few warps (100 x
-// 300: 92 against 121 us; at 2,048 143 each).
-constexpr int64_t kFewGeneric = 1024;
-// swift_sw_batch: from here on (pairs, and query rows in all) the packed
-// passes are faster (2,048 pairs of 36 x 100: 66 us on the int32 kernel, 77
-// packed; 4,096: 92 each; 2,048 of 100 x 300: 143 each; 2,048 of 250 x 500:
-// 511 against 306; 1,024 of 250 x 500: 271 against 290).
-constexpr int64_t kBatchPackedPairs = 2048, kBatchPackedRows = 200000;
+// Of these, pairs in this range all run on the int32 kernel: its warp a pair
+// holds directions in shared memory and walks them there, so it ends before
+// the packed trace pass and walk, two launches of a few warps (2,000 reads of
+// 100 bases 391 against 412 us, 4,000 of 50 385 against 408).  Fewer pairs
+// seldom hold one with other bytes, which alone takes the int32 kernel its
+// whole 55 us, beside 40 and 13 (300 reads 313 against 300 us).
+constexpr int64_t kFewGenericMin = 100, kFewGeneric = 1024;
+// swift_sw_batch: whether the packed passes are the faster ones.  The int32
+// kernel's time grows with the pairs past its resident warps, that of the
+// packed passes with the rows' chain of steps first (us, int32 / packed: 2,048
+// pairs of 36 x 100 64 / 70, 4,096 90 / 82; 1,536 of 100 x 300 114 / 121, 2,048
+// 141 / 127; 1,024 of 200 x 300 143 / 147, 1,536 208 / 172; 512 of 250 x 500
+// 146 / 184, 1,024 270 / 190).
+bool batch_packed(int64_t n, int Q) {
+  const int64_t rows = n * Q;
+  return rows >= 250000 || (n >= 2048 && rows >= 200000) || (n >= 4096 && rows >= 140000);
+}
 // swift_sw_pairs: its launches alternate between two streams from here on
 constexpr int64_t kAlternatePairs = 1024;
 // and classes of fewer pairs than kMergePairs share a launch; launches of
@@ -1475,13 +1482,12 @@ int swift_sw_batch(swift_ctx* ctx, const char* qry, const char* ref, int32_t Q, 
   a.qcons = dqc;
   a.rcons = drc;
   a.cons_stride = cs;
-  // From kBatchPackedPairs and -Rows on, pairs of bases run on the packed trace
-  // pass and walk, in chunks that bound its scratch; the others, and every
+  // Where they are the faster (batch_packed), pairs of bases run on the packed
+  // trace pass and walk, in chunks that bound its scratch; the others, and every
   // pair where the scoring or that scratch is not to be had, on the int32
   // kernel, which needs none.
   int bias = 0;
-  bool packed = n >= kBatchPackedPairs && n * Q >= kBatchPackedRows &&
-                fast_params_ok(Q, R, m, x, o, e, &bias);
+  bool packed = batch_packed(n, Q) && fast_params_ok(Q, R, m, x, o, e, &bias);
   const int64_t chunk = std::min<int64_t>(n, 131072);
   BatchArgs ba;
   FastArgs fa;
@@ -2496,8 +2502,8 @@ static int align_resident_impl(swift_ctx* ctx, const swift_index* idx, const swi
     }
   }
   // few records: each traced at once (see kDirectPairs); else bounded selection
-  // (below kFewGeneric on the int32 kernel alone)
-  if (ctx->sw_path == 0 && n <= kFewGeneric) fast_ok = false;
+  // (from kFewGenericMin to kFewGeneric on the int32 kernel alone)
+  if (ctx->sw_path == 0 && n > kFewGenericMin && n <= kFewGeneric) fast_ok = false;
   const bool direct = fast_ok && ctx->sw_path == 0 && !sam && n <= kDirectPairs;
   const bool bounded = fast_ok && ctx->sw_path == 0 && !sam && !direct;
   const int Qs = (Q + 16) & ~15;
@@ -3514,7 +3520,7 @@ static int align_paired_impl(swift_ctx* ctx, const swift_index* idx, const char*
   pl.q_stride = qs;
   pl.w_stride = ws;
   // few records left: all on the int32 kernel (kFewGeneric)
-  if (left_n <= kFewGeneric) fast_ok = false;
+  if (left_n > kFewGenericMin && left_n <= kFewGeneric) fast_ok = false;
   launch_pe_pairs(st, pl);
   CKLAUNCH();
   launches += left_n > 0 ? 1 : 0;

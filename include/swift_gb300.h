@@ -94,8 +94,8 @@ typedef struct {
                             (there the printed ones)                         */
   int64_t bound_pruned;  /* pairs whose score bound ruled them out, so they
                             needed no exact score                            */
-  int64_t retraced_pairs;/* printed pairs traced after selection (bounded
-                            selection: the read's candidate was not best)    */
+  int64_t retraced_pairs;/* printed pairs traced after their read's candidate
+                            (bounded selection: it was not best)             */
   double first_pass_ms;  /* the packed path's first kernel alone: the LCS
                             bound (default) or the exact score pass; 0 where
                             every pair is traced (SAM output, small calls)   */

@@ -405,7 +405,15 @@ __global__ void aln_to_ref_layout_kernel(const DevAln* __restrict__ aln, int64_t
 // costs less than the passes, lists and host round trips that would spare
 // most of them: at these sizes each pass lasts as long as one pair does.
 constexpr int64_t kDirectPairs = 3072;
-// Of these, pairs in this range all run on the int32 kernel: its warp a pair
+// With more, pairs the LCS bound keeps are traced at once up to this many query
+// rows, and only scored, with a second trace of the printed ones, beyond: the
+// second trace is a launch chain and a host round trip of its own, the cells a
+// score would not compute cost more from here on (scored and traced again
+// against traced: 2,036 pairs of 251 rows 926 / 840 us a call, 4,255 of 100
+// 639 / 600, 12,899 of 60 910 / 875, 8,704 of 150 1,269 / 1,222; 17,052 of 100
+// 1,202 / 1,216, 40,002 1,804 / 1,902).
+constexpr int64_t kTraceKeptRows = 1500000;
+// Of kDirectPairs, those in this range all run on the int32 kernel: its warp a pair
 // holds directions in shared memory and walks them there, so it ends before
 // the packed trace pass and walk, two launches of a few warps (2,000 reads of
 // 100 bases 391 against 412 us, 4,000 of 50 385 against 408).  Fewer pairs
@@ -2803,6 +2811,7 @@ static int align_resident_impl(swift_ctx* ctx, const swift_index* idx, const swi
     if (rc != SWIFT_OK) return rc;
   }
   int64_t lcs_kept = 0, cand_n = 0;
+  bool trace_kept = false;  // the kept pairs were traced, not only scored
   if (bounded && n > 0) {
     // candidates (largest LCS bound of their group) traced first; they stop
     // early on the LCS pass's suffix values, in an order that groups pairs
@@ -2853,14 +2862,20 @@ static int align_resident_impl(swift_ctx* ctx, const swift_index* idx, const swi
         if (rc != SWIFT_OK) return rc;
         ex_list = sorted;
       }
-      fa2.list = ex_list;
-      fa2.count = cnt + 3;
-      fa2.list_offset = 0;
-      few_pairs_shape(Q, lcs_kept, &fa2.shape_g, &fa2.shape_rpl);
-      fa2.cand = cand;
-      launches += launch_sw_score(st, fa2, lcs_kept);
-      CKLAUNCH();
-      fa2.cand = nullptr;
+      trace_kept = lcs_kept * Q <= kTraceKeptRows;
+      if (trace_kept) {
+        rc = trace_list(ex_list, cnt + 3, lcs_kept, false);
+        if (rc != SWIFT_OK) return rc;
+      } else {
+        fa2.list = ex_list;
+        fa2.count = cnt + 3;
+        fa2.list_offset = 0;
+        few_pairs_shape(Q, lcs_kept, &fa2.shape_g, &fa2.shape_rpl);
+        fa2.cand = cand;
+        launches += launch_sw_score(st, fa2, lcs_kept);
+        CKLAUNCH();
+        fa2.cand = nullptr;
+      }
     }
   }
   if (generic.armed) {
@@ -2880,7 +2895,7 @@ static int align_resident_impl(swift_ctx* ctx, const swift_index* idx, const swi
         pairs, keep, cand, n, fast_ok && !direct ? 0 : 1, list2, cnt + 4, cnt + 5);
     CKLAUNCH();
     ++launches;
-    if (fast_ok && !direct) {
+    if (fast_ok && !direct && !trace_kept) {
       CK(rb.get(h_cnt, cnt, sizeof(h_cnt)));
       CK(rb.sync());
       rc = trace_list(list2, cnt + 4, h_cnt[4], false);
@@ -3002,7 +3017,7 @@ static int align_resident_impl(swift_ctx* ctx, const swift_index* idx, const swi
     s.seed_overflow_strands = so.overflow;
     s.printed = sam ? nproc : h_cnt[5] + settled[1];
     s.sw_generic_pairs = h_cnt[1];
-    s.traced_pairs = sam ? h_cnt[0] + settled[0] : (direct ? h_cnt[0] : h_cnt[2] + h_cnt[4]) + settled[1];
+    s.traced_pairs = sam ? h_cnt[0] + settled[0] : (direct ? h_cnt[0] : h_cnt[2] + (trace_kept ? lcs_kept : h_cnt[4])) + settled[1];
     s.bound_pruned = pruned + (sam ? 0 : settled[0] - settled[1]);
     s.retraced_pairs = bounded ? h_cnt[4] : 0;
     // build_pairs + the Smith-Waterman passes and select (launches) +

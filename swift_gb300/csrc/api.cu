@@ -101,6 +101,14 @@ struct Scratch {
     }
     return cudaSuccess;
   }
+  // Gives a request of `bytes` back before the call's end, in stream order
+  // (one cut from a shared block stays).
+  void drop(void* p, size_t bytes) {
+    const auto it = std::find(ptrs.begin(), ptrs.end(), p);
+    if (bytes <= kCarve || it == ptrs.end()) return;
+    cudaFreeAsync(p, st);
+    ptrs.erase(it);
+  }
 };
 
 // Small device values the host waits for.  A copy to pageable memory holds
@@ -2189,17 +2197,36 @@ int swift_sw_pairs(swift_ctx* ctx, const char* qry, const int64_t* q_off, const 
         CK(sc.get(&doff, (size_t)n_long));
         CK(cudaMemcpyAsync(dlist, ids.data(), n_long * 4, cudaMemcpyHostToDevice, st));
         CK(cudaMemcpyAsync(doff, off.data(), n_long * 8, cudaMemcpyHostToDevice, st));
-        const int n_regions = batches.size() > 1 ? 2 : 1;
-        // whole GiB, so that calls of like sizes find the pool's block again
-        // (a new size maps memory anew, 1.3 ms at 4 GB)
+        // Whole GiB, so that calls of like sizes find the pool's block again
+        // (a new size maps memory anew, 1.3 ms at 4 GB); the exact size where
+        // that is not to be had, then with the packed launches' regions
+        // (joined above) given back.
         constexpr int64_t kGiB = 1 << 28;
-        if (max_words > kGiB) max_words = (max_words + kGiB - 1) & ~(kGiB - 1);
-        for (int r = 0; r < n_regions; ++r) {
-          if (max_words > dirs_words[r]) {
-            CK(sc.get(&dirs[r], (size_t)max_words));
-            dirs_words[r] = max_words;
+        auto region = [&](int r) -> cudaError_t {
+          if (max_words <= dirs_words[r]) return cudaSuccess;
+          for (int t = max_words > kGiB ? 0 : 1;; ++t) {
+            const int64_t w = t == 0 ? (max_words + kGiB - 1) & ~(kGiB - 1) : max_words;
+            const cudaError_t e = sc.get(&dirs[r], (size_t)w);
+            if (e == cudaSuccess) {
+              dirs_words[r] = w;
+              return e;
+            }
+            cudaGetLastError();
+            if (t == 2 || (t == 1 && r > 0)) return e;
+            if (t == 1) {
+              for (int q = 0; q < 2; ++q) {
+                sc.drop(dirs[q], (size_t)dirs_words[q] * sizeof(uint32_t));
+                dirs_words[q] = 0;
+              }
+              cudaMemPool_t pool;
+              cudaStreamSynchronize(st);
+              if (cudaDeviceGetMemPool(&pool, ctx->device) == cudaSuccess) cudaMemPoolTrimTo(pool, 0);
+            }
           }
-        }
+        };
+        CK(region(0));
+        // (no memory for a second region: the launches one after another)
+        const int n_regions = batches.size() > 1 && region(1) == cudaSuccess ? 2 : 1;
         if (n_regions > 1) {
           const int rc = side_fork(ctx);
           if (rc != SWIFT_OK) return rc;
@@ -2207,7 +2234,8 @@ int swift_sw_pairs(swift_ctx* ctx, const char* qry, const int64_t* q_off, const 
         }
         for (size_t b = 0; b < batches.size(); ++b) {
           const LongBatch& lb = batches[b];
-          cudaStream_t bs = (b & 1) ? ctx->side : st;
+          const int r = n_regions > 1 ? (int)(b & 1) : 0;
+          cudaStream_t bs = r ? ctx->side : st;
           LongArgs la;
           memset(&la, 0, sizeof(la));
           la.qry = dq;
@@ -2223,7 +2251,7 @@ int swift_sw_pairs(swift_ctx* ctx, const char* qry, const int64_t* q_off, const 
           la.mismatch = x;
           la.gap_open = o;
           la.gap_ext = e;
-          la.dirs = dirs[b & 1];
+          la.dirs = dirs[r];
           la.dir_off = doff + lb.b0;
           la.best = best2;
           la.aln = aln;

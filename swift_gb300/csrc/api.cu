@@ -47,6 +47,8 @@ int index_global_positions(swift_index* ix, cudaStream_t st) {
 namespace {
 
 int fail(swift_ctx* ctx, int code, const std::string& msg) {
+  // (reported here: the thread's next call does not take it for its own)
+  if (code == SWIFT_E_CUDA) cudaGetLastError();
   if (ctx) ctx->err = msg;
   return code;
 }

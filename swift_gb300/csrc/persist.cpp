@@ -69,6 +69,7 @@ struct Checksum {
 };
 
 int fail(swift_ctx* ctx, int code, const std::string& msg) {
+  if (code == SWIFT_E_CUDA) cudaGetLastError();  // reported here
   if (ctx) ctx->err = msg;
   return code;
 }

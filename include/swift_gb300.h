@@ -100,7 +100,9 @@ typedef struct {
                             bound (default) or the exact score pass; 0 where
                             every pair is traced (SAM output, small calls)   */
   int64_t first_pass_cells; /* DP cells that kernel covered               */
-  int64_t first_pass_kind;  /* 1 exact score, 3 LCS bound, 0 none         */
+  int64_t first_pass_kind;  /* 1 exact score (also of the int32 kernel, with
+                            path 1 or scoring the packed passes do not take),
+                            3 LCS bound, 0 none                            */
   double trace_ms;       /* trace-pass launches: the candidates (default;
                             they stop early on suffix LCS values) or every
                             packed pair over whole windows (SAM)            */

@@ -2541,7 +2541,8 @@ static int align_resident_impl(swift_ctx* ctx, const swift_index* idx, const swi
   }
   // few records: each traced at once (see kDirectPairs); else bounded selection
   // (from kFewGenericMin to kFewGeneric on the int32 kernel alone)
-  if (ctx->sw_path == 0 && n > kFewGenericMin && n <= kFewGeneric) fast_ok = false;
+  const bool few_generic = fast_ok && ctx->sw_path == 0 && n > kFewGenericMin && n <= kFewGeneric;
+  if (few_generic) fast_ok = false;
   const bool direct = fast_ok && ctx->sw_path == 0 && !sam && n <= kDirectPairs;
   const bool bounded = fast_ok && ctx->sw_path == 0 && !sam && !direct;
   const int Qs = (Q + 16) & ~15;
@@ -3020,11 +3021,11 @@ static int align_resident_impl(swift_ctx* ctx, const swift_index* idx, const swi
     }
     s.trace_ms = trace_sum;
     s.trace_cells = (int64_t)h_cells2[1];
-    if (!sam) {
+    if (!sam && !direct && !few_generic) {
       cudaEventElapsedTime(&t, ctx->ev[7], ctx->ev[8]);
       s.first_pass_ms = t;
-      s.first_pass_kind = direct ? 0 : bounded ? 3 : 1;
-      s.first_pass_cells = fast_ok && !direct ? (int64_t)h_cnt[0] * Q * kWin : 0;
+      s.first_pass_kind = bounded ? 3 : 1;
+      s.first_pass_cells = fast_ok ? (int64_t)h_cnt[0] * Q * kWin : 0;
     }
     s.lcs_kept = lcs_kept;
     s.seed_kernel_ms = so.kernel_ms;

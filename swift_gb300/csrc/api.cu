@@ -423,13 +423,28 @@ constexpr int64_t kDirectPairs = 3072;
 // 639 / 600, 12,899 of 60 910 / 875, 8,704 of 150 1,269 / 1,222; 17,052 of 100
 // 1,202 / 1,216, 40,002 1,804 / 1,902).
 constexpr int64_t kTraceKeptRows = 1500000;
-// Of kDirectPairs, those in this range all run on the int32 kernel: its warp a pair
-// holds directions in shared memory and walks them there, so it ends before
-// the packed trace pass and walk, two launches of a few warps (2,000 reads of
-// 100 bases 391 against 412 us, 4,000 of 50 385 against 408).  Fewer pairs
-// seldom hold one with other bytes, which alone takes the int32 kernel its
-// whole 55 us, beside 40 and 13 (300 reads 313 against 300 us).
-constexpr int64_t kFewGenericMin = 100, kFewGeneric = 1024;
+// Whether so few records, of queries of Q rows, all run on the int32 kernel: its
+// warp a pair holds directions in shared memory and walks them there, so it
+// can end before the packed trace pass and walk, two launches of a few warps.
+// Fewer than kFewGenericMin seldom hold a pair with other bytes, which alone
+// takes the int32 kernel its whole 55 us, beside 40 and 13.  A step of either
+// costs its rows per lane, in the int32 kernel a 32nd of the query:
+//   to 128 rows four on both sides; within 30 us either way (us, int32 /
+//     packed: 608 pairs of 50 rows 377 / 409, 504 of 100 327 / 316, 892 368 / 383)
+//   to 224 seven on both sides and the packed passes are the faster (364 of
+//     200 359 / 330, 677 of 129 396 / 341)
+//   to 256 eight against sixteen, as long as each pair has a scheduler to
+//     itself (407 of 240 335 / 354, 737 374 / 356)
+//   beyond, ten on both sides (502 of 300 331 / 304, 854 465 / 345).
+// lcs_first: the packed route opens with the LCS pass and two waits for it (SAM
+// output of reads cut off by their windows: 554 of 205 367 / 432, 1,024 of 240
+// 413 / 488, 602 of 300 415 / 479, 854 497 / 472).
+constexpr int64_t kFewGenericMin = 100, kFewGeneric = 1024, kOnePerScheduler = 4 * 152;
+bool few_on_int32(int64_t n, int Q, bool lcs_first) {
+  if (n <= kFewGenericMin || n > kFewGeneric) return false;
+  if (Q <= 128 || (lcs_first && Q <= 256)) return true;
+  return n <= kOnePerScheduler && (lcs_first || (Q > 224 && Q <= 256));
+}
 // swift_sw_batch: whether the packed passes are the faster ones.  The int32
 // kernel's time grows with the pairs past its resident warps, that of the
 // packed passes with the rows' chain of steps first (us, int32 / packed: 2,048
@@ -2540,8 +2555,8 @@ static int align_resident_impl(swift_ctx* ctx, const swift_index* idx, const swi
     }
   }
   // few records: each traced at once (see kDirectPairs); else bounded selection
-  // (from kFewGenericMin to kFewGeneric on the int32 kernel alone)
-  const bool few_generic = fast_ok && ctx->sw_path == 0 && n > kFewGenericMin && n <= kFewGeneric;
+  // (or all on the int32 kernel)
+  const bool few_generic = fast_ok && ctx->sw_path == 0 && few_on_int32(n, Q, sam && cut_reads);
   if (few_generic) fast_ok = false;
   const bool direct = fast_ok && ctx->sw_path == 0 && !sam && n <= kDirectPairs;
   const bool bounded = fast_ok && ctx->sw_path == 0 && !sam && !direct;
@@ -3565,8 +3580,9 @@ static int align_paired_impl(swift_ctx* ctx, const swift_index* idx, const char*
   pl.wbuf = wbuf;
   pl.q_stride = qs;
   pl.w_stride = ws;
-  // few records left: all on the int32 kernel (kFewGeneric)
-  if (left_n > kFewGenericMin && left_n <= kFewGeneric) fast_ok = false;
+  // (mates of 150 bases, calls of 250 pairs 497 us on the int32 kernel, 463 packed,
+  // of 1,000 712 / 667; of 100 bases, 1,800 537 / 581)
+  if (few_on_int32(left_n, Q, false)) fast_ok = false;
   launch_pe_pairs(st, pl);
   CKLAUNCH();
   launches += left_n > 0 ? 1 : 0;

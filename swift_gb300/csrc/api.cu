@@ -1925,6 +1925,7 @@ int swift_sw_pairs(swift_ctx* ctx, const char* qry, const int64_t* q_off, const 
         bool gen;
         int Q, R;           // generic: the shape; packed: the class's rows, widest window
         int64_t start, count;
+        int low;            // packed: the rows of the lowest class that shares the launch
       };
       std::vector<Group> groups;
       std::vector<std::pair<int64_t, int64_t>> long_groups;  // (start, count) per rows class
@@ -1948,7 +1949,7 @@ int swift_sw_pairs(swift_ctx* ctx, const char* qry, const int64_t* q_off, const 
           groups.back().count += hc[s];
           continue;
         }
-        groups.push_back({gen, gen ? q : 8 * q, R, hs[s], hc[s]});
+        groups.push_back({gen, gen ? q : 8 * q, R, hs[s], hc[s], 8 * q});
       }
       ps.segments += (int64_t)groups.size();
       // launch sizes go to the device (the kernels read counts there)
@@ -1962,7 +1963,10 @@ int swift_sw_pairs(swift_ctx* ctx, const char* qry, const int64_t* q_off, const 
       const int64_t sub = 262144;
       // a class's (lanes, rows per lane) shape: the default (0, 0), a forced
       // candidate, or the fastest candidate on a sample of these pairs
-      // (timed once per context, class and window bin)
+      // (timed once per context, range of classes and window bin; a launch of
+      // several classes takes the choice of its tallest alone, but not the
+      // other way round: its sample is a mix)
+      auto tuned_key = [](int low, const Group& G) { return ((low / 8) * 64 + G.Q / 8) * 64 + (G.R + 63) / 64; };
       struct Plan {
         int bias = 0, g = 0, rpl = 0;
         bool tune = false;
@@ -1987,7 +1991,8 @@ int swift_sw_pairs(swift_ctx* ctx, const char* qry, const int64_t* q_off, const 
         if (ctx->tuning == 1 && G.count < kTunePairs) {
           few_pairs_shape(G.Q, G.count, &pl.g, &pl.rpl);
         } else if (ctx->tuning == 1) {
-          auto it = ctx->tuned.find((G.Q / 8) * 64 + (G.R + 63) / 64);
+          auto it = ctx->tuned.find(tuned_key(G.low, G));
+          if (it == ctx->tuned.end()) it = ctx->tuned.find(tuned_key(G.Q, G));
           if (it != ctx->tuned.end()) {
             pl.g = it->second.first;
             pl.rpl = it->second.second;
@@ -2044,9 +2049,10 @@ int swift_sw_pairs(swift_ctx* ctx, const char* qry, const int64_t* q_off, const 
         int32_t cg[16], crpl[16];
         const int ncand = packed_shape_candidates(G.Q, cg, crpl, 16);
         if (pl.tune) {
-          // a sample from the middle of the class (its pairs are sorted by
-          // window length), each candidate launched once on a few of them
-          // (its code loaded) and timed once
+          // a sample from the middle of the launch (sorted by class, then
+          // window length; the classes below the tallest hold fewer than
+          // kMergePairs), each candidate launched once on a few of them (its
+          // code loaded) and timed once
           const int64_t ns = std::min<int64_t>(G.count, 16384);
           int32_t* ns_d;
           CK(sc.get(&ns_d, 1));
@@ -2079,7 +2085,7 @@ int swift_sw_pairs(swift_ctx* ctx, const char* qry, const int64_t* q_off, const 
               best = c;
             }
           }
-          ctx->tuned[(G.Q / 8) * 64 + (G.R + 63) / 64] = {cg[best], crpl[best]};
+          ctx->tuned[tuned_key(G.low, G)] = {cg[best], crpl[best]};
           pl.g = cg[best];
           pl.rpl = crpl[best];
         }

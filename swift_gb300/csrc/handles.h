@@ -33,7 +33,7 @@ struct swift_ctx {
   // swift_sw_pairs: 1 autotune the packed shape per (query class, window
   // bin), 0 default shapes, k >= 2 the (k-2)-th candidate of every class
   int tuning = 1;
-  std::map<int, std::pair<int, int>> tuned;  // (class, window bin) -> (lanes, rows per lane)
+  std::map<int, std::pair<int, int>> tuned;  // (classes, window bin) -> (lanes, rows per lane)
 };
 
 struct swift_index {

@@ -3324,7 +3324,6 @@ static int align_paired_impl(swift_ctx* ctx, const swift_index* idx, const char*
   CK(sc.get(&pa.m_rev, nr));
   CK(sc.get(&pa.m_read, nr));
   CK(sc.get(&pa.m_ri, nr));
-  CK(sc.get(&pa.m_shift, nr));
   CK(sc.get(&pa.m_off, nr));
   pa.roff = roff;
   pa.n_rec = (int64_t)nrec;

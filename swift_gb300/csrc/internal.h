@@ -405,7 +405,7 @@ struct PairedArgs {
   const int3 *best1, *best2;
   const uint64_t* roff;       // per pair: first record
   int64_t n_rec;
-  int32_t *m_id, *m_rev, *m_read, *m_ri, *m_shift, *m_off;  // m_read: mate 2's after mate 1's
+  int32_t *m_id, *m_rev, *m_read, *m_ri, *m_off;  // m_read: mate 2's after mate 1's
   int Q;
   const char* ref_file;
   uint64_t ref_file_len;
@@ -422,8 +422,6 @@ struct PairedArgs {
 void launch_pe_records(cudaStream_t st, const PairedArgs& a, uint64_t* cnt);
 void launch_pe_fill(cudaStream_t st, const PairedArgs& a);
 void launch_pe_pairs(cudaStream_t st, const PairedArgs& a);
-void launch_aln_from_arrays(cudaStream_t st, const float* score, const int32_t* start,
-                            const int32_t* end, const int32_t* len, int64_t n, DevAln* aln);
 void launch_shift_reads(cudaStream_t st, const DevRead* in, int64_t n, uint64_t by,
                         DevRead* out);
 // mate pairing (chooseBestAlignment_paired3) and printOutput_paired2 flags

@@ -39,7 +39,6 @@ __global__ void pe_fill_kernel(PairedArgs a) {
         a.m_rev[o] = s;
         a.m_read[o] = (int32_t)(mate * a.n_pairs + i);
         a.m_ri[o] = b.x;
-        a.m_shift[o] = b.y;
         a.m_off[o] = b.z;
         ++o;
       }
@@ -153,21 +152,6 @@ __global__ void __launch_bounds__(kPeWarps * 32) pe_pairs_kernel(PairedArgs a) {
     p.flags = (odd || got != R) ? 1 : 0;
     a.pairs[j] = p;
   }
-}
-
-__global__ void aln_from_arrays_kernel(const float* __restrict__ score,
-                                       const int32_t* __restrict__ start,
-                                       const int32_t* __restrict__ end,
-                                       const int32_t* __restrict__ len, int64_t n,
-                                       DevAln* __restrict__ aln) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  DevAln d;
-  d.score = (int32_t)score[i];
-  d.start = start[i];
-  d.end = end[i];
-  d.len = len[i];
-  aln[i] = d;
 }
 
 // the second reads file's records after the first's: offsets shifted by the
@@ -377,13 +361,6 @@ void launch_pe_fill(cudaStream_t st, const PairedArgs& a) {
 void launch_pe_pairs(cudaStream_t st, const PairedArgs& a) {
   if (a.n_rec <= 0) return;
   pe_pairs_kernel<<<(unsigned)((a.n_rec + kPeWarps - 1) / kPeWarps), kPeWarps * 32, 0, st>>>(a);
-}
-
-void launch_aln_from_arrays(cudaStream_t st, const float* score, const int32_t* start,
-                            const int32_t* end, const int32_t* len, int64_t n, DevAln* aln) {
-  if (n <= 0) return;
-  aln_from_arrays_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(score, start, end, len, n,
-                                                                       aln);
 }
 
 void launch_pe_runs(cudaStream_t st, const PairSelArgs& a, uint32_t* flag) {

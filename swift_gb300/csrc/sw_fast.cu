@@ -185,11 +185,8 @@ int packed_shape_candidates(int Q, int32_t* g, int32_t* rpl, int cap) {
 }
 
 int launch_sw_score(cudaStream_t st, const FastArgs& a, int64_t max_pairs) {
-  FastArgs b = a;
-  b.one = 1;
-  b.four = 4;
-  return a.q_len ? launch_shape<false, true>(st, b, max_pairs)
-                 : launch_shape<false, false>(st, b, max_pairs);
+  return a.q_len ? launch_shape<false, true>(st, a, max_pairs)
+                 : launch_shape<false, false>(st, a, max_pairs);
 }
 
 int launch_sw_trace(cudaStream_t st, const FastArgs& a, int64_t max_pairs, cudaEvent_t before,

@@ -439,10 +439,13 @@ constexpr int64_t kTraceKeptRows = 1500000;
 // lcs_first: the packed route opens with the LCS pass and two waits for it (SAM
 // output of reads cut off by their windows: 554 of 205 367 / 432, 1,024 of 240
 // 413 / 488, 602 of 300 415 / 479, 854 497 / 472).
+// wave: a server's wave runs beside other workers' waves, where one launch is the
+// cheaper whatever the rows (48 requests of 50 to 300 bases on four workers 5.48
+// / 5.56 ms).
 constexpr int64_t kFewGenericMin = 100, kFewGeneric = 1024, kOnePerScheduler = 4 * 152;
-bool few_on_int32(int64_t n, int Q, bool lcs_first) {
+bool few_on_int32(int64_t n, int Q, bool lcs_first, bool wave) {
   if (n <= kFewGenericMin || n > kFewGeneric) return false;
-  if (Q <= 128 || (lcs_first && Q <= 256)) return true;
+  if (wave || Q <= 128 || (lcs_first && Q <= 256)) return true;
   return n <= kOnePerScheduler && (lcs_first || (Q > 224 && Q <= 256));
 }
 // swift_sw_batch: whether the packed passes are the faster ones.  The int32
@@ -1966,7 +1969,9 @@ int swift_sw_pairs(swift_ctx* ctx, const char* qry, const int64_t* q_off, const 
       // (timed once per context, range of classes and window bin; a launch of
       // several classes takes the choice of its tallest alone, but not the
       // other way round: its sample is a mix)
-      auto tuned_key = [](int low, const Group& G) { return ((low / 8) * 64 + G.Q / 8) * 64 + (G.R + 63) / 64; };
+      auto tuned_key = [](int low, const Group& G) {
+        return ((low / 8) * 64 + G.Q / 8) * 64 + (G.R + 63) / 64;
+      };
       struct Plan {
         int bias = 0, g = 0, rpl = 0;
         bool tune = false;
@@ -2562,7 +2567,7 @@ static int align_resident_impl(swift_ctx* ctx, const swift_index* idx, const swi
   }
   // few records: each traced at once (see kDirectPairs); else bounded selection
   // (or all on the int32 kernel)
-  const bool few_generic = fast_ok && ctx->sw_path == 0 && few_on_int32(n, Q, sam && cut_reads);
+  const bool few_generic = fast_ok && ctx->sw_path == 0 && few_on_int32(n, Q, sam && cut_reads, wave);
   if (few_generic) fast_ok = false;
   const bool direct = fast_ok && ctx->sw_path == 0 && !sam && n <= kDirectPairs;
   const bool bounded = fast_ok && ctx->sw_path == 0 && !sam && !direct;
@@ -3587,7 +3592,7 @@ static int align_paired_impl(swift_ctx* ctx, const swift_index* idx, const char*
   pl.w_stride = ws;
   // (mates of 150 bases, calls of 250 pairs 497 us on the int32 kernel, 463 packed,
   // of 1,000 712 / 667; of 100 bases, 1,800 537 / 581)
-  if (few_on_int32(left_n, Q, false)) fast_ok = false;
+  if (few_on_int32(left_n, Q, false, false)) fast_ok = false;
   launch_pe_pairs(st, pl);
   CKLAUNCH();
   launches += left_n > 0 ? 1 : 0;

@@ -230,6 +230,14 @@ int swift_sw_batch_noalloc(swift_ctx *ctx, const char *qry, const char *ref, int
                            int32_t *start, int32_t *end, int32_t *len, char *qcons,
                            char *rcons);
 
+/* Scratch of swift_sw_batch and swift_sw_pairs.  Both take direction scratch from
+ * the device's stream-ordered memory pool, which keeps it for later calls:
+ * swift_sw_batch for up to 131,072 pairs at a time on the packed passes (1.3 GB
+ * at 100 x 300, 9.1 GB at 320 x 512; without it the pairs run on the int32
+ * kernel, which needs none), swift_sw_pairs two regions for up to 262,144 pairs
+ * each and for long pairs two of up to 8 GiB (one where there is no memory for
+ * two).  A caller that shares the GPU gives the memory back between calls with
+ * cudaMemPoolTrimTo. */
 /* Statistics of one swift_sw_pairs call. */
 typedef struct {
   double ms;               /* device time of the call (CUDA events)           */

@@ -290,9 +290,13 @@ __global__ void __launch_bounds__(kLT, 2) sw_long_kernel(LongArgs a) {
 // final maximum is never missed, since the warp's largest so far never
 // exceeds it.
 //
-// Per two cells 12.5 instructions, 6.5 on the ALU pipe, where the int32
-// kernel takes 28 and 18 (500 pairs of 1-4 kb by 2-8 kb: 3.5 ms, 13.4 before
-// over four launches).
+// Per two cells of a strip 12.5 instructions, 6.5 on the ALU pipe, where the
+// int32 kernel takes 28 and 18 (500 pairs of 1-4 kb by 2-8 kb: 3.5 ms, 13.4
+// before over four launches).  Over a whole launch 19.5 and 10.1 per two cells of
+// the pairs (300 of them, one wave): the step's shuffles, ring, selectors and
+// tests are shared by 4 to 16 rows, and rows past the query and skewed columns
+// count too.  The ALU pipe is busy 56 % of the time; the largest stall is the
+// barrier between stages, where warps that have not started or have ended wait.
 constexpr int kStage16 = 16;
 constexpr int kLag16 = 5;    // stages between neighbouring warps
 constexpr int kRing16 = 64;  // ring columns

@@ -31,9 +31,9 @@
 // Layout: one thread per record; the codes of the reference (16 bases a
 // word, in L2) and of the reads, both strands, are read in place, so no
 // window or query is written out for the records this settles.  Bound by
-// the ALU pipe (84 %): at 100-base reads and 300-base windows about 2,000
-// instructions a record, against 190,000 for the trace pass's share of a pair
-// (4.13 M records 0.56 ms).
+// the ALU pipe (88 %): at 100-base reads and 300-base windows a warp takes 3,600
+// instructions for its 32 records, 2,500 of them on that pipe (4.13 M records
+// 0.56 ms).
 //
 // gapless_bound_kernel applies the same argument with a smaller bound to the
 // pairs that remain, once the LCS pass has run: the matches of a chain are a

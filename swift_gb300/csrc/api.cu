@@ -2826,7 +2826,7 @@ static int align_resident_impl(swift_ctx* ctx, const swift_index* idx, const swi
       CK(rb.sync());
       int32_t *sam_list = fast_list, *sam_count = cnt;
       int64_t sam_traced = h_cnt[0];
-      if (lsuf) {
+      if (lsuf && h_cnt[0] > 0) {  // (all pairs can be the int32 kernel's)
         // suffix LCS values for the early stop, then the order that groups
         // pairs stopping alike
         fa2.list = fast_list;

@@ -93,3 +93,17 @@ def test_reads_file_sizes(ctx, oracle, size):
     for t in (text, text[:-1]):
         want = oracle.align(fa, t, oracle.default_params(device_mem=ctx.info()["total_mem"]))
         assert len(want) > 900 and ctx.align(ix, t) == want
+
+
+@pytest.mark.parametrize("L", [100, 204, 205, 250])
+@pytest.mark.parametrize("fmt", [0, 1])
+def test_no_packed_pair(ctx, sg, L, fmt):
+    # windows cut short by their sequence's end: every pair is the int32 kernel's
+    rng = random.Random(L)
+    seqs = [bytes(rng.choice(b"ACGT") for _ in range(L + 40)) for _ in range(3)]
+    reads = b"".join(b">r%d\n%s\n" % (i, seqs[i % 3][i:i + L]) for i in range(30))
+    ix = ctx.index(test_gapless.fasta(seqs))
+    p = sg.default_params(max_read_len=300, out_format=fmt)
+    got, st = ctx.align(ix, reads, p, stats=True)
+    assert st["sw_generic_pairs"] == st["records"] >= 30
+    assert got == by_int32(ctx, lambda: ctx.align(ix, reads, p))

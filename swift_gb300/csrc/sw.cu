@@ -233,11 +233,13 @@ constexpr size_t kGenericSmemMax = 200 * 1024;
 template <int RPL, int W, bool CODED>
 int launch_generic_w(cudaStream_t st, const SwArgs& a, int pw) {
   const size_t smem = (size_t)pw * W;
-  // the opt-in above 48 KB is a per-device function attribute: set it on
-  // every launch (cheap), so a second device or context needs no state here
+  // The opt-in above 48 KB is a per-device function attribute: set on every
+  // launch (cheap), so a second device or context needs no state here, and
+  // always to the most, since another thread's launch may come between.
   if (smem > 48 * 1024 &&
       cudaFuncSetAttribute(sw_generic_kernel<RPL, W, CODED>,
-                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+                           cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)kGenericSmemMax) != cudaSuccess)
     return SWIFT_E_CUDA;
   int64_t blocks = (a.n + W - 1) / W;
   if (a.list) {  // the list's length is on the device: a few waves stride over it

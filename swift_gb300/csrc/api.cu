@@ -1105,7 +1105,8 @@ int swift_ctx_create(int device, void* stream, swift_ctx** out) {
   for (int i = 0; i < kCtxEvents && e == cudaSuccess; ++i) e = cudaEventCreate(&ctx->ev[i]);
   if (e == cudaSuccess) e = cudaMallocHost(&ctx->mail, kMailBytes);
   if (e != cudaSuccess) {
-    delete ctx;
+    swift_ctx_destroy(ctx);
+    cudaGetLastError();  // reported here, as in fail()
     return SWIFT_E_CUDA;
   }
   keep_pool(device);
@@ -1129,7 +1130,7 @@ int swift_ctx_destroy(swift_ctx* ctx) {
   }
   for (cudaEvent_t e : ctx->chunk_ev) cudaEventDestroy(e);
   for (cudaEvent_t e : ctx->copy_ev) cudaEventDestroy(e);
-  if (ctx->own_stream) cudaStreamDestroy(ctx->st);
+  if (ctx->own_stream && ctx->st) cudaStreamDestroy(ctx->st);
   delete ctx;
   return SWIFT_OK;
 }

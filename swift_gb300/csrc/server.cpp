@@ -365,7 +365,10 @@ int swift_server_create(int device, const swift_index* idx, const swift_params* 
       p->max_hits > 64 || (p->seeder != 0 && p->seeder != 1) || p->max_read_len < 0 ||
       p->max_read_len > kSeedReadMax)
     return SWIFT_E_ARG;
-  if (cudaSetDevice(device) != cudaSuccess) return SWIFT_E_CUDA;
+  if (cudaSetDevice(device) != cudaSuccess) {
+    cudaGetLastError();  // reported here
+    return SWIFT_E_CUDA;
+  }
   swift_server* s = new swift_server();
   s->device = device;
   s->idx = idx;
@@ -374,6 +377,7 @@ int swift_server_create(int device, const swift_index* idx, const swift_params* 
     size_t fr = 0, tot = 0;
     if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) {
       delete s;
+      cudaGetLastError();
       return SWIFT_E_CUDA;
     }
     mem_budget = (int64_t)(fr / 2);

@@ -1,5 +1,5 @@
-"""A call that fails for want of memory leaves nothing behind: the next call of
-the same context gives its own result."""
+"""A call that fails, for want of memory or of the device it names, leaves nothing
+behind: the thread's next call gives its own result."""
 import random
 
 import numpy as np
@@ -31,3 +31,21 @@ def test_call_after_out_of_memory(kind):
         with pytest.raises(sg.SwiftError):
             call()
     assert call() == want
+
+
+def test_call_after_a_device_that_is_not_there():
+    from swift_gb300 import build as b
+    b.build()
+    import swift_gb300 as sg
+    rng = random.Random(4)
+    ref = bytes(rng.choice(b"ACGT") for _ in range(3000))
+    ctx = sg.Context(0)
+    ix = ctx.index(b">chr\n" + ref + b"\n")
+    reads = b">r\n" + ref[500:600] + b"\n"
+    want = ctx.align(ix, reads)
+    with pytest.raises(sg.SwiftError):
+        sg.Context(4096)
+    assert ctx.align(ix, reads) == want
+    with pytest.raises(sg.SwiftError):
+        sg.Server(ix, 4096)
+    assert ctx.align(ix, reads) == want
